@@ -336,14 +336,11 @@ int stage_batch_new(const std::vector<FockPlan *> &plans, const std::vector<doub
     }
     for (int gi : groups) di.push_back(make_int4(m, gi, 0, 0));
     const int npad = scr ? p->nblocks64 * 16 : (int)padded_points(N);
-    int chunk = 0;
-    const int nchunk =
-        npad > 0 ? quadrature_chunking(p->n, npad, &chunk, (int)padded_points(N)) : 0;
-    const int nblk = (p->n + 127) / 128, ntile = nblk * (nblk + 1) / 2;
+    const QuadPlan plan = quad_plan(p->n, npad);  // no kept point: no chunk, F = 0
     qa[m] = QuadBatchArg{p->phi.p, p->ld, b->wv.p + b->offp[m], p->work.p, F[m],
-                         scr ? p->blocks64.p : nullptr, p->n, npad, nblk, chunk, nchunk};
-    for (int c = 0; c < nchunk; ++c)
-      for (int t = 0; t < ntile; ++t) qi.push_back(make_int4(m, t, c, 0));
+                         scr ? p->blocks64.p : nullptr, p->n, npad, plan};
+    const int nitem = quad_plan_items(p->n, plan);
+    for (int c = 0; c < nitem; ++c) qi.push_back(make_int4(m, c, 0, 0));
     wa[m] = WeightBatchArg{p->grid->dev.wb, p->grid->dev.w, b->v.p + b->off[m],
                            b->wv.p + b->offp[m], N, (int)p->ld};
   }

@@ -50,14 +50,24 @@ struct DensBatchArg {      // density of one molecule
   const int *keep;         // screening flags or null
   int n, npoint, vecD, pad;
 };
+// Split of an FP64 quadrature into partial sums (quad_plan in quad.cu).
+// n <= 64: class 0 holds nch[0] chunks of chunk[0] points, one warp each.
+// n > 64: the 128 x 128 tiles of the upper triangle in four classes of equal
+// cost (right of the diagonal: full, last column; diagonal: full, last); class
+// c has ntile[c] tiles, each split into nch[c] chunks of chunk[c] points, its
+// CTAs numbered from first[c], tile fastest; CTA b writes workspace slot b.
+struct QuadPlan {
+  int ntile[4], nch[4], chunk[4], first[5];
+};
 struct QuadBatchArg {      // quadrature of one molecule
   const double *phi;       // [n][ld]
   long ld;
   const double *wv;        // zero padded to npoint rounded up to 128
-  double *work;            // [nchunk][tile][128][128]
+  double *work;            // partial sums (QuadPlan)
   double *F;               // [n][n]
   const int *blocks;       // 16-point blocks of a screened plan, or null
-  int n, npad, nblk, chunk, nchunk;
+  int n, npad;
+  QuadPlan plan;
 };
 struct WeightBatchArg {    // wv = wb w (q v), zero padded to npad
   const double *wb, *w, *v;
@@ -65,7 +75,7 @@ struct WeightBatchArg {    // wv = wb w (q v), zero padded to npad
   int npoint, npad;
 };
 // Device work queue of a persistent batched launch: items[i] = (molecule,
-// tile, chunk, -); item i is taken once *posted > i, waiting at most
+// group or CTA, -, -); item i is taken once *posted > i, waiting at most
 // timeout_ns; a timeout records kDeviceTimeout in *status.
 struct BatchQueue {
   const int4 *items;
@@ -75,9 +85,11 @@ struct BatchQueue {
   int *status;
   unsigned long long timeout_ns;
 };
-// Split-K chunking of a K range of npad points in a workspace sized for a grid
-// of pad_full points (quadrature_workspace_bytes): chunk count <= the grid's.
-int quadrature_chunking(int n, int npad, int *chunk, int pad_full);
+// Plan of a K range of npad points; fits the workspace of every grid of at
+// least npad points (quadrature_workspace_bytes).
+QuadPlan quad_plan(int n, int npad);
+// Work items of a batched quadrature: a CTA each (n > 64) or 8 chunks (n <= 64).
+int quad_plan_items(int n, const QuadPlan &p);
 cudaError_t launch_density_batch(const DensBatchArg *args, const BatchQueue &q, int grid,
                                  cudaStream_t s);
 cudaError_t launch_quadrature_batch(const QuadBatchArg *args, const BatchQueue &q, int grid,
@@ -95,11 +107,6 @@ inline long padded_points(int npoint) { return ((long)npoint + 127) / 128 * 128;
 cudaError_t launch_combine_weights(int npoint, const double *wb, const double *w,
                                    double q, const double *v, const double *vext,
                                    double *wv, cudaStream_t s);
-
-// Adds nchunk partial 128x128 upper-triangle tiles [chunk][tile][128][128]
-// in fixed order and writes both triangles of F.
-cudaError_t launch_quadrature_reduce(int n, int nchunk, const double *work, double *F,
-                                     cudaStream_t s);
 
 // Int8-slice tensor-core quadratures (tc.cu).  A plan holds phi's operand
 // images (built once from phi, wb and w) and the per-call scratch; the calls

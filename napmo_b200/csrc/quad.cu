@@ -10,25 +10,42 @@
 // Psi[n(n+1)/2][N] (src/wavefunction/nwavefunction.cpp:77-107,161-197).  Here
 // both are FP64 GEMMs over phi stored basis-major [n][ld] (ld a multiple of
 // 128, zero padded), issued as mma.sync m16n8k8 f64 (DMMA: 2048 flops per
-// warp instruction, FP64 accumulation) from operand tiles that cp.async
-// streams into a 4-stage shared-memory ring:
+// warp instruction, FP64 accumulation).  Both are bound by the FP64 tensor
+// pipe (64 FMA per clock and SM, one m16n8k8 per 64 clocks and sub-partition;
+// a cuBLAS DGEMM of 8192^3 reaches 35.5 TFLOP/s), so what counts is that no
+// instruction is spent on entries nobody needs: work is dropped in 16 x 8
+// (quadrature) and 16 x 16 (density) fragments, below the diagonal and beyond
+// the last basis function.
 //
-//   * density: a CTA owns 128 points and sweeps 128-row blocks of mu.  D is
-//     folded onto block-upper-triangular form (block b of mu takes nu from
-//     its own first row on; entries right of the diagonal block count twice,
-//     exact for symmetric D), so the CTA forms T' = D' phi for each block
-//     (62 % of the full product at n = 510) and folds T' into the per-point
-//     sum with phi[mu][p] in the epilogue; deterministic, no atomics.
-//   * quadrature: split-K over points.  CTA (tile, chunk) accumulates one
-//     128x128 upper-triangle tile of F over one chunk of points into a
-//     workspace slot (wv applied to the B fragments in registers); a second
-//     kernel adds the chunks in fixed order and writes both triangles, so F
-//     is exactly symmetric and bit-reproducible.
+//   * n <= 64 (kSmallN): every warp holds the whole upper triangle of
+//     fragments and works on its own points, straight from global memory to
+//     registers; the CTA's 8 warps are summed in shared memory (quadrature).
+//     With 128-wide tiles a 25-function molecule spent 16 % of a tile's
+//     fragments, and wrote 128 x 128 partial sums per chunk (77 MB).
+//   * n > 64: 128 x 128 tiles per CTA from a 4-stage cp.async ring, 8 warps
+//     as 2 x 4, each 4 x 4 fragments interleaved over the tile (rows 16 (wr +
+//     2 mt), columns 8 (wc + 4 nt)), so that the fragments left of a diagonal
+//     or ragged tile are spread over the four sub-partitions.
 //
-// Tiles: 128x128 per CTA, 8 warps as 2 x 4 of 64x32 (4 x 4 m16n8 tiles, 64
-// FP64 accumulators per thread), 16 points (quadrature) or 16 functions
-// (density) per stage.  Shared-memory rows are padded to a stride of 4 mod 16
-// doubles, so the fragment loads of each half-warp hit 16 distinct banks.
+// density: D is folded onto block-upper-triangular form at 16 x 16 (row tile i
+// takes nu from its own first row on; entries right of its diagonal block
+// count twice, exact for symmetric D); T' = D' phi is folded into the
+// per-point sum with phi[mu][p] as soon as a row tile is complete;
+// deterministic, no atomics.
+// quadrature: split-K over points; chunk partials go to a workspace and a
+// second kernel adds them in a fixed order and writes both triangles, so F is
+// exactly symmetric and bit-reproducible.
+//
+// Shared-memory rows are padded to a stride of 4 mod 16 doubles, so the
+// fragment loads of each half-warp hit 16 distinct banks.
+//
+// Measured (B200, 1965 MHz; before: whole 128 x 128 tiles for every n):
+//   density     H2O (25 functions, 16,500 points)          8.2 ->  4.0 us
+//               C12H26 (310 functions, 1,147,600 points)  6.25 -> 4.62 ms
+//   quadrature  H2O, both kernels                           87 ->   11 us
+//               C8H18 (210 functions, 785,200 points)     2.63 -> 1.78 ms
+//               C12H26                                    7.51 -> 5.30 ms
+#include <algorithm>
 #include <cstdint>
 #include <string>
 
@@ -79,55 +96,159 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// acc[mt][nt] += A-tile rows (warp rows mt) x B-tile columns (warp columns nt)
-// over one stage: A fragments from a[row][k], B fragments from bf(col, k).
-template <typename BFrag>
-__device__ __forceinline__ void stage_mma(const double (*a)[LDA], int wrow, int g, int q,
-                                          BFrag bf, double (&acc)[4][4][4]) {
+constexpr int kSmallN = 64;            // whole triangle of fragments per warp up to this n
+constexpr int kWarps = NT / 32;
+// row tiles of 16 that cover n <= kSmallN, and their upper-triangle fragments
+__host__ __device__ constexpr int small_tiles(int n) { return (n + 15) / 16; }
+__host__ __device__ constexpr int small_frags(int rt) { return rt * (rt + 1); }
+
+// ------------------------------------------------------------------ density
+// n <= 64: T'[i] = D'[i] phi for 8 points, rho = sum of T' phi.  A warp keeps
+// the fragments of D' (row tile i, k8 step kk >= 2 i; entries right of the
+// diagonal 16 x 16 block doubled) in registers for all its points.
+template <int RT>
+__device__ __forceinline__ void density_small_frags(int n, const double *__restrict__ D,
+                                                    double (&a)[RT * (RT + 1)][4]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  int f = 0;
 #pragma unroll
-  for (int kk = 0; kk < BK; kk += 8) {
-    double b[4][2];
+  for (int i = 0; i < RT; ++i)
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt) bf(nt, kk, b[nt]);
+    for (int kk = 2 * i; kk < 2 * RT; ++kk, ++f)
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt) {
-      const int r = wrow + mt * 16 + g;
-      const double af[4] = {a[r][kk + q], a[r + 8][kk + q], a[r][kk + q + 4],
-                            a[r + 8][kk + q + 4]};
+      for (int c = 0; c < 4; ++c) {
+        const int mu = 16 * i + g + 8 * (c & 1), nu = 8 * kk + q + 4 * (c >> 1);
+        const double d = mu < n && nu < n ? __ldg(D + (long)mu * n + nu) : 0.0;
+        a[f][c] = kk >= 2 * i + 2 ? 2.0 * d : d;
+      }
+}
+
+template <int RT>
+__device__ __forceinline__ void density_small_points(const double (&a)[RT * (RT + 1)][4], int n,
+                                                     int npoint, const double *__restrict__ phi,
+                                                     long ld, double *__restrict__ rho, int p0,
+                                                     const int *__restrict__ keep) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  double b[2 * RT][2];
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt], af, b[nt]);
+  for (int kk = 0; kk < 2 * RT; ++kk)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int nu = 8 * kk + q + 4 * h;
+      b[kk][h] = nu < n ? __ldg(phi + (long)nu * ld + p0 + g) : 0.0;
+    }
+  double2 fr[RT][2];  // phi[mu] of the accumulator's rows and columns
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int mu = 16 * i + g + 8 * h;
+      fr[i][h] = mu < n ? __ldg(reinterpret_cast<const double2 *>(phi + (long)mu * ld + p0 + 2 * q))
+                        : make_double2(0.0, 0.0);
+    }
+  double s0 = 0.0, s1 = 0.0;
+  int f = 0;
+#pragma unroll
+  for (int i = 0; i < RT; ++i) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int kk = 2 * i; kk < 2 * RT; ++kk, ++f) dmma(acc, a[f], b[kk]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      s0 = fma(acc[2 * h], fr[i][h].x, s0);
+      s1 = fma(acc[2 * h + 1], fr[i][h].y, s1);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {
+    s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+  }
+  if (g < 2) {  // lane (g, q) writes point 2 q + g
+    const int p = p0 + 2 * q + g;
+    if (p < npoint) rho[p] = (keep && !keep[p]) ? 0.0 : (g ? s1 : s0);
+  }
+}
+
+// The 128-point groups bx, bx + gx, ... of `ngroup` (listed in `groups`, or
+// all): warp w takes points 16 w .. 16 w + 15 of each.
+template <int RT>
+__device__ __forceinline__ void density_small_block(int n, int npoint,
+                                                    const double *__restrict__ phi, long ld,
+                                                    const double *__restrict__ D,
+                                                    double *__restrict__ rho,
+                                                    const int *__restrict__ groups, int ngroup,
+                                                    int bx, int gx,
+                                                    const int *__restrict__ keep) {
+  double a[RT * (RT + 1)][4];
+  density_small_frags<RT>(n, D, a);
+  const int warp = threadIdx.x >> 5;
+  for (int gi = bx; gi < ngroup; gi += gx) {
+    const int p0 = (groups ? groups[gi] : gi) * BN + 16 * warp;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      density_small_points<RT>(a, n, npoint, phi, ld, rho, p0 + 8 * h, keep);
+  }
+}
+
+__device__ __forceinline__ void density_small_any(int n, int npoint,
+                                                  const double *__restrict__ phi, long ld,
+                                                  const double *__restrict__ D,
+                                                  double *__restrict__ rho,
+                                                  const int *__restrict__ groups, int ngroup,
+                                                  int bx, int gx, const int *__restrict__ keep) {
+  switch (small_tiles(n)) {
+    case 1: density_small_block<1>(n, npoint, phi, ld, D, rho, groups, ngroup, bx, gx, keep); break;
+    case 2: density_small_block<2>(n, npoint, phi, ld, D, rho, groups, ngroup, bx, gx, keep); break;
+    case 3: density_small_block<3>(n, npoint, phi, ld, D, rho, groups, ngroup, bx, gx, keep); break;
+    default: density_small_block<4>(n, npoint, phi, ld, D, rho, groups, ngroup, bx, gx, keep);
+  }
+}
+
+template <int RT>
+__global__ void __launch_bounds__(NT)
+density_small_kernel(int n, int npoint, const double *__restrict__ phi, long ld,
+                     const double *__restrict__ D, double *__restrict__ rho,
+                     const int *__restrict__ groups, int ngroup, const int *__restrict__ keep) {
+  density_small_block<RT>(n, npoint, phi, ld, D, rho, groups, ngroup, blockIdx.x, gridDim.x,
+                          keep);
+}
+
+// n > 64.  Stages of a CTA: block mb of mu takes nu from mb*BM to n (rounded up
+// to BK = 16), the blocks one after the other; within a block the nu right of
+// the diagonal block come first and the diagonal block's own nu last, in
+// descending order, so that row tile i (16 rows) takes every stage before its
+// own one doubled, its own once, and none after it.  Its phi rows are then in
+// the stage's shared memory, where the fold into rho reads them.
+struct DensStage {
+  int mb, k0;
+  int diag;  // the stage's row tile within the diagonal block, or 8 right of it
+};
+__device__ __forceinline__ void density_stage_next(DensStage &s, int nk) {
+  constexpr int SB = BM / BK;                      // stages per 128 functions
+  const int k = s.k0 / BK;
+  if (s.diag == SB) {                              // right of the diagonal block
+    if (k + 1 < nk) {
+      s.k0 += BK;
+    } else {
+      s.diag = SB - 1;                             // a full block: others lie right of it
+      s.k0 = (s.mb * SB + s.diag) * BK;
+    }
+  } else if (s.diag > 0) {
+    --s.diag;
+    s.k0 -= BK;
+  } else {
+    ++s.mb;
+    if ((s.mb + 1) * SB < nk) {
+      s.diag = SB;
+      s.k0 = (s.mb + 1) * SB * BK;
+    } else {
+      s.diag = min(SB, nk - s.mb * SB) - 1;
+      s.k0 = (s.mb * SB + s.diag) * BK;
     }
   }
 }
 
-// ------------------------------------------------------------------ density
-// Stages of a CTA: block mb of mu takes nu from mb*BM to n (rounded up to BK),
-// the blocks one after the other; within a block the nu right of the
-// diagonal block come first and the diagonal block's own nu last, so the
-// doubling of the off-diagonal part is one multiply of the accumulators
-// before the first diagonal stage.  Returns k0 of stage `it` and sets its
-// block, whether it is the block's first diagonal stage, and whether it is
-// the block's last stage.
-__device__ __forceinline__ int density_stage(int it, int nblk, int nk, int &mb, bool &first_diag,
-                                             bool &last) {
-  constexpr int SB = BM / BK;                   // stages per 128 functions
-  mb = 0;
-  int left = it;
-  while (mb < nblk) {
-    const int cnt = nk - mb * SB;
-    if (left < cnt) break;
-    left -= cnt;
-    ++mb;
-  }
-  const int ndiag = min(SB, nk - mb * SB);      // diagonal-block stages
-  const int noff = nk - mb * SB - ndiag;        // stages right of it
-  last = left == noff + ndiag - 1;
-  first_diag = left == noff;
-  return left < noff ? ((mb + 1) * SB + left) * BK : (mb * SB + left - noff) * BK;
-}
-
-// groups (optional): the 128-point groups to compute (screened plans; the
-// others hold no kept point); keep (optional): rho = 0 at dropped points.
 // rho of the 128 points p0 .. p0 + 127 (one CTA; see density_kernel).
 template <bool kVecD>
 __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
@@ -135,43 +256,41 @@ __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
                                               const double *__restrict__ D,
                                               double *__restrict__ rho, int p0,
                                               const int *__restrict__ keep) {
+  constexpr int SB = BM / BK;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int g = lane >> 2, q = lane & 3;
-  const int wrow = (warp >> 2) * 64, wcol = (warp & 3) * 32;
+  const int wr = warp >> 2, wcol = (warp & 3) * 32;
   const int nblk = (n + BM - 1) / BM;
   const int nk = (n + BK - 1) / BK;                 // stages of nu over the whole basis
   int nstage = 0;
-  for (int mb = 0; mb < nblk; ++mb) nstage += nk - mb * (BM / BK);
+  for (int mb = 0; mb < nblk; ++mb) nstage += nk - mb * SB;
 
   // copies of one stage: D' rows (16-byte copies when n is even and D is
-  // 16-byte aligned, else 8-byte) and phi rows (16-byte copies; p0 + c is
-  // even, ld even)
-  auto load_stage = [&](int it) {
-    int mb;
-    bool fd, ls;
-    const int k0 = density_stage(it, nblk, nk, mb, fd, ls);
-    const int slot = it % NS;
+  // 16-byte aligned, else 8-byte; in a diagonal stage only the row tiles that
+  // still take it) and phi rows (16-byte copies; p0 + c is even, ld even)
+  auto load_stage = [&](const DensStage &st, int slot) {
+    const int rows = st.diag == SB ? BM : 16 * (st.diag + 1);
     if (kVecD) {
 #pragma unroll
       for (int i = 0; i < (BM * BK / 2) / NT; ++i) {
         const int e = t + NT * i, r = e / (BK / 2), c = (e % (BK / 2)) * 2;
-        const int mu = mb * BM + r, nu = k0 + c;
+        const int mu = st.mb * BM + r, nu = st.k0 + c;
         const bool v = mu < n && nu < n;   // n even: nu + 1 < n as well
-        cp_async16(&sm.a[slot][r][c], D + (v ? (long)mu * n + nu : 0), v);
+        if (r < rows) cp_async16(&sm.a[slot][r][c], D + (v ? (long)mu * n + nu : 0), v);
       }
     } else {
 #pragma unroll
       for (int i = 0; i < (BM * BK) / NT; ++i) {
         const int e = t + NT * i, r = e / BK, c = e % BK;
-        const int mu = mb * BM + r, nu = k0 + c;
+        const int mu = st.mb * BM + r, nu = st.k0 + c;
         const bool v = mu < n && nu < n;
-        cp_async8(&sm.a[slot][r][c], D + (v ? (long)mu * n + nu : 0), v);
+        if (r < rows) cp_async8(&sm.a[slot][r][c], D + (v ? (long)mu * n + nu : 0), v);
       }
     }
 #pragma unroll
     for (int i = 0; i < (BK * BN / 2) / NT; ++i) {
       const int e = t + NT * i, r = e / (BN / 2), c = (e % (BN / 2)) * 2;
-      const int nu = k0 + r;
+      const int nu = st.k0 + r;
       const bool v = nu < n;
       cp_async16(&sm.b[slot][r][c], phi + (v ? (long)nu * ld + p0 + c : 0), v);
     }
@@ -188,61 +307,77 @@ __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.0;
 
+  DensStage ld_st{-1, 0, 0}, st{-1, 0, 0};
+  density_stage_next(ld_st, nk);
+  density_stage_next(st, nk);
 #pragma unroll
   for (int i = 0; i < NS - 1; ++i) {
-    if (i < nstage) load_stage(i);
+    if (i < nstage) {
+      load_stage(ld_st, i);
+      density_stage_next(ld_st, nk);
+    }
     cp_async_commit();
   }
   for (int it = 0; it < nstage; ++it) {
     cp_async_wait<NS - 2>();
     __syncthreads();
-    if (it + NS - 1 < nstage) load_stage(it + NS - 1);
-    cp_async_commit();
-    int mb;
-    bool first_diag, last;
-    density_stage(it, nblk, nk, mb, first_diag, last);
+    auto next_copies = [&] {
+      if (it + NS - 1 < nstage) {
+        load_stage(ld_st, (it + NS - 1) % NS);
+        density_stage_next(ld_st, nk);
+      }
+      cp_async_commit();
+    };
+    // half of each sub-partition's warps issue the copies before their
+    // products, the other half after the first ones: its pipe does not idle
+    if (wr == 0) next_copies();
     const int slot = it % NS;
-    if (first_diag) {
-      // the part right of the diagonal block counts twice (D symmetric)
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) acc[mt][nt][i] *= 2.0;
-    }
+    const double(*at)[LDA] = sm.a[slot];
     const double(*bt)[LDB] = sm.b[slot];
-    stage_mma(sm.a[slot], wrow, g, q,
-              [&](int nt, int kk, double(&b)[2]) {
-                const int c = wcol + nt * 8 + g;
-                b[0] = bt[kk + q][c];
-                b[1] = bt[kk + q + 4][c];
-              },
-              acc);
-    // last stage of block mb: part[p] += sum_mu T'[mu][p] phi[mu][p]
-    if (last) {
+    const int left = nk - st.mb * SB;             // row tiles of the block
+    double b[2][4][2];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+    for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int mu = mb * BM + wrow + mt * 16 + g + 8 * h;
-          if (mu < n) {
-            const double *prow = phi + (long)mu * ld + p0 + wcol + 2 * q;
+      for (int nt = 0; nt < 4; ++nt) {
+        const int c = wcol + nt * 8 + g;
+        b[kk][nt][0] = bt[8 * kk + q][c];
+        b[kk][nt][1] = bt[8 * kk + q + 4][c];
+      }
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-              const double2 f = __ldg(reinterpret_cast<const double2 *>(prow + nt * 8));
-              part[nt][0] = fma(acc[mt][nt][2 * h], f.x, part[nt][0]);
-              part[nt][1] = fma(acc[mt][nt][2 * h + 1], f.y, part[nt][1]);
-            }
-          }
-        }
-#pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+    for (int mt = 0; mt < 4; ++mt) {
+      if (wr == 1 && mt == 1) next_copies();
+      const int i = wr + 2 * mt;                  // row tile within the block
+      if (i > st.diag || i >= left) continue;     // warp-uniform
+      if (i == st.diag) {
+        // the part right of the row tile's diagonal block counts twice
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-          for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.0;
+          for (int c = 0; c < 4; ++c) acc[mt][nt][c] *= 2.0;
+      }
+      const int r = 16 * i + g;
+#pragma unroll
+      for (int kk = 0; kk < 2; ++kk) {
+        const double af[4] = {at[r][8 * kk + q], at[r + 8][8 * kk + q], at[r][8 * kk + q + 4],
+                              at[r + 8][8 * kk + q + 4]};
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt], af, b[kk][nt]);
+      }
+      if (i == st.diag) {  // complete: part[p] += sum_mu T'[mu][p] phi[mu][p]
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            const double2 f =
+                *reinterpret_cast<const double2 *>(&bt[g + 8 * h][wcol + nt * 8 + 2 * q]);
+            part[nt][0] = fma(acc[mt][nt][2 * h], f.x, part[nt][0]);
+            part[nt][1] = fma(acc[mt][nt][2 * h + 1], f.y, part[nt][1]);
+            acc[mt][nt][2 * h] = acc[mt][nt][2 * h + 1] = 0.0;
+          }
+      }
     }
+    density_stage_next(st, nk);
   }
   cp_async_wait<0>();
   // sum over the warp's rows (lanes of equal q), then over the two warp rows
@@ -268,6 +403,8 @@ __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
     rho[p0 + t] = (keep && !keep[p0 + t]) ? 0.0 : sm.red[0][t] + sm.red[1][t];
 }
 
+// groups (optional): the 128-point groups to compute (screened plans; the
+// others hold no kept point); keep (optional): rho = 0 at dropped points.
 template <bool kVecD>
 __global__ void __launch_bounds__(NT, 1)
 density_kernel(int n, int npoint, const double *__restrict__ phi, long ld,
@@ -284,33 +421,140 @@ density_kernel(int n, int npoint, const double *__restrict__ phi, long ld,
 // points); with it (screened plans) the K range is the list of 16-point
 // blocks holding a kept point, npoint_pad = 16 x their count and `chunk` a
 // multiple of 16 as before.
-// Tile `tile` (upper-triangle index) of F over chunk `ck` of the points into
-// its workspace slot (one CTA; see quadrature_kernel).
+
+// n <= 64: each warp accumulates the whole upper triangle of 16 x 8 fragments
+// over a chunk of its own; the B fragments of the second operand psi = phi are
+// A fragments times the weights (A's rows g and g + 8 are B's columns of two
+// fragments), so one set of loads feeds both.  Sums run over the points of a
+// chunk and then over the chunks in order.
+template <int RT, bool kSame>
+__device__ __forceinline__ void quadrature_small_chunk(int n, int npoint_pad,
+                                                       const double *__restrict__ phi,
+                                                       const double *__restrict__ phib, long ld,
+                                                       const double *__restrict__ wv, int chunk,
+                                                       double *__restrict__ work,
+                                                       const int *__restrict__ blocks, int ck) {
+  constexpr int T = small_frags(RT);
+  const int lane = threadIdx.x & 31;
+  const int g = lane >> 2, q = lane & 3;
+  const int s_begin = ck * (chunk / 8), s_end = min((ck + 1) * chunk, npoint_pad) / 8;
+  if (s_begin >= s_end) return;
+  double acc[T][4];
+#pragma unroll
+  for (int f = 0; f < T; ++f)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[f][c] = 0.0;
+  // rows 16 i + g, 16 i + 8 + g of an operand at points p0 + q, p0 + q + 4
+  auto load = [&](const double *x, long p0, double (&f)[RT][4]) {
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int r = 16 * i + g + 8 * (c & 1);
+        f[i][c] = r < n ? __ldg(x + (long)r * ld + p0 + q + 4 * (c >> 1)) : 0.0;
+      }
+  };
+#pragma unroll (RT <= 2 ? 4 : RT == 3 ? 2 : 1)
+  for (int s = s_begin; s < s_end; ++s) {
+    const long p0 = blocks ? (long)blocks[s >> 1] * BK + (s & 1) * 8 : 8L * s;
+    const double w0 = __ldg(wv + p0 + q), w1 = __ldg(wv + p0 + q + 4);
+    double a[RT][4], b[RT][4];
+    load(phi, p0, a);
+    if (!kSame) load(phib, p0, b);
+#pragma unroll
+    for (int i = 0; i < RT; ++i) {
+      b[i][0] = (kSame ? a[i][0] : b[i][0]) * w0;
+      b[i][1] = (kSame ? a[i][1] : b[i][1]) * w0;
+      b[i][2] = (kSame ? a[i][2] : b[i][2]) * w1;
+      b[i][3] = (kSame ? a[i][3] : b[i][3]) * w1;
+    }
+    int f = 0;
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int j = 2 * i; j < 2 * RT; ++j, ++f) {
+        const double bf[2] = {b[j >> 1][j & 1], b[j >> 1][2 + (j & 1)]};
+        dmma(acc[f], a[i], bf);
+      }
+  }
+  double *out = work + (long)ck * (T * 128) + lane;
+#pragma unroll
+  for (int f = 0; f < T; ++f)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) out[f * 128 + c * 32] = acc[f][c];
+}
+
+template <int RT>
+__global__ void __launch_bounds__(NT)
+quadrature_small_kernel(int n, int npoint_pad, const double *__restrict__ phi,
+                        const double *__restrict__ phib, long ld,
+                        const double *__restrict__ wv, int chunk, double *__restrict__ work,
+                        const int *__restrict__ blocks) {
+  const int ck = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (phi == phib)
+    quadrature_small_chunk<RT, true>(n, npoint_pad, phi, phib, ld, wv, chunk, work, blocks, ck);
+  else
+    quadrature_small_chunk<RT, false>(n, npoint_pad, phi, phib, ld, wv, chunk, work, blocks, ck);
+}
+
+// n > 64.  Tile `t` of class `c` (QuadPlan) of nblk x nblk blocks.
+__device__ __forceinline__ void quad_tile(int c, int t, int nblk, int &mb, int &nb) {
+  if (c == 0) {
+    nb = 1;
+    while (t >= nb) t -= nb++;
+    mb = t;
+  } else if (c == 1) {
+    mb = t;
+    nb = nblk - 1;
+  } else {
+    mb = nb = c == 2 ? t : nblk - 1;
+  }
+}
+
+// Fragments of one warp in a diagonal tile of R row tiles (16 rows) and C = 2 R
+// or 2 R - 1 column tiles (8 columns).  Row tile i has the C - 2 i fragments
+// from column 2 i on; row tiles p and R - 1 - p together have twice L = C - R
+// + 1, so warp 2 p takes the first L of row p and warp 2 p + 1 the rest of it
+// and all of row R - 1 - p (for odd R the middle row is warp R - 1's alone):
+// R warps of L fragments each.
+struct DiagFrags {
+  int r0, r1;      // row tiles of the fragments [0, split) and [split, count)
+  int c0, c1;      // their first column tiles
+  int split, count;
+};
+__device__ __forceinline__ DiagFrags diag_frags(int R, int C, int warp) {
+  const int L = C - R + 1, p = warp >> 1, last = R - 1 - p;
+  if (warp >= R) return DiagFrags{0, 0, 0, 0, 0, 0};
+  if ((warp & 1) == 0) return DiagFrags{p, p, 2 * p, 2 * p, L, L};
+  return DiagFrags{p, last, 2 * p + L, 2 * last, R - 1 - 2 * p, L};
+}
+
+// CTA `cta` of the plan: one tile of F over one chunk of the points, into its
+// workspace slot.  Only the 16 x 8 fragments that hold an entry of the upper
+// triangle within n are multiplied and written; they are skipped by branches
+// around groups of instructions (a predicated-off DMMA still takes its slot in
+// the pipe: masking single fragments gained nothing).
 __device__ __forceinline__ void quadrature_block(QuadSmem &sm, int n, int npoint_pad,
                                                  const double *__restrict__ phi,
                                                  const double *__restrict__ phib, long ld,
-                                                 const double *__restrict__ wv, int nblk,
-                                                 int chunk, double *__restrict__ work,
-                                                 const int *__restrict__ blocks, int tile_index,
-                                                 int ck) {
+                                                 const double *__restrict__ wv,
+                                                 const QuadPlan &plan,
+                                                 double *__restrict__ work,
+                                                 const int *__restrict__ blocks, int cta) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int g = lane >> 2, q = lane & 3;
-  const int wrow = (warp >> 2) * 64, wcol = (warp & 3) * 32;
-  // upper-triangle tile index -> (mb, nb)
-  int tile = tile_index, mb = 0;
-  {
-    int rem = tile;
-    while (rem >= nblk - mb) {
-      rem -= nblk - mb;
-      ++mb;
-    }
-    tile = rem;  // offset within row mb
-  }
-  const int nb = mb + tile;
+  int cls = 0;
+  while (cta >= plan.first[cls + 1]) ++cls;
+  const int local = cta - plan.first[cls], ck = local / plan.ntile[cls];
+  const int chunk = plan.chunk[cls];
+  int mb, nb;
+  quad_tile(cls, local - ck * plan.ntile[cls], (n + BM - 1) / BM, mb, nb);
   const int mu0 = mb * BM, nu0 = nb * BN;
+  const bool same = mb == nb && phi == phib;       // one operand tile serves both
   const int k_begin = ck * chunk;
   const int k_end = min(k_begin + chunk, npoint_pad);
   const int nstage = k_end > k_begin ? (k_end - k_begin) / BK : 0;
+  const int ncol = (min(n - nu0, BN) + 7) / 8;     // live column tiles
 
   // copies of one stage: 128 rows x 16 points of each operand (8 x 16 bytes
   // per row) and the 16 weights; rows beyond n are zero filled
@@ -322,87 +566,225 @@ __device__ __forceinline__ void quadrature_block(QuadSmem &sm, int n, int npoint
       const int e = t + NT * i, r = e / (BK / 2), c = (e % (BK / 2)) * 2;
       const bool va = mu0 + r < n, vb = nu0 + r < n;
       cp_async16(&sm.a[slot][r][c], phi + (va ? (long)(mu0 + r) * ld + k0 + c : 0), va);
-      cp_async16(&sm.b[slot][r][c], phib + (vb ? (long)(nu0 + r) * ld + k0 + c : 0), vb);
+      if (!same)
+        cp_async16(&sm.b[slot][r][c], phib + (vb ? (long)(nu0 + r) * ld + k0 + c : 0), vb);
     }
     if (t < BK / 2) cp_async16(&sm.w[slot][2 * t], wv + k0 + 2 * t, true);
   };
-
-  double acc[4][4][4];
-#pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[mt][nt][i] = 0.0;
-
+  // one stage's turn: the stage's data is in, the next copies are issued (by
+  // half of the warps before their products, by the other half of each
+  // sub-partition's after the first ones, so that its pipe does not idle)
+  auto begin_stage = [&](int it) {
+    cp_async_wait<NS - 2>();
+    __syncthreads();
+    if (warp < 4) {
+      if (it + NS - 1 < nstage) load_stage(it + NS - 1);
+      cp_async_commit();
+    }
+  };
+  auto mid_stage = [&](int it) {
+    if (warp >= 4) {
+      if (it + NS - 1 < nstage) load_stage(it + NS - 1);
+      cp_async_commit();
+    }
+  };
 #pragma unroll
   for (int i = 0; i < NS - 1; ++i) {
     if (i < nstage) load_stage(i);
     cp_async_commit();
   }
+  double *out = work + (long)cta * (BM * BN);
+  auto store = [&](int r, int c, const double(&v)[4]) {
+    double *o = out + (16 * r + g) * BN + 8 * c + 2 * q;
+    *reinterpret_cast<double2 *>(o) = make_double2(v[0], v[1]);
+    *reinterpret_cast<double2 *>(o + 8 * BN) = make_double2(v[2], v[3]);
+  };
+
+  if (mb == nb) {
+    constexpr int F = 9;                           // most fragments of a warp (R = 8)
+    const int R = (min(n - mu0, BM) + 15) / 16;
+    const DiagFrags d = diag_frags(R, ncol, warp);
+    double acc[F][4];
+    int bo[F];                                     // row of the B tile of fragment f
+#pragma unroll
+    for (int f = 0; f < F; ++f) {
+      bo[f] = 8 * (f < d.split ? d.c0 + f : d.c1 + f - d.split) + g;
+      if (f >= d.count) bo[f] = g;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[f][c] = 0.0;
+    }
+    for (int it = 0; it < nstage; ++it) {
+      begin_stage(it);
+      const int slot = it % NS;
+      const double(*at)[LDA] = sm.a[slot];
+      const double(*bt)[LDA] = same ? sm.a[slot] : sm.b[slot];
+      const double *w = sm.w[slot];
+#pragma unroll
+      for (int kk = 0; kk < BK; kk += 8) {
+        const double w0 = w[kk + q], w1 = w[kk + q + 4];
+        const double *x0 = &at[16 * d.r0 + g][kk + q], *x1 = &at[16 * d.r1 + g][kk + q];
+        const double a0[4] = {x0[0], x0[8 * LDA], x0[4], x0[8 * LDA + 4]};
+        const double a1[4] = {x1[0], x1[8 * LDA], x1[4], x1[8 * LDA + 4]};
+#pragma unroll
+        for (int f3 = 0; f3 < F; f3 += 3) {
+          if (f3 >= d.count) continue;             // warp-uniform
+#pragma unroll
+          for (int f = f3; f < f3 + 3; ++f) {
+            const double b[2] = {bt[bo[f]][kk + q] * w0, bt[bo[f]][kk + q + 4] * w1};
+            const bool lo = f < d.split;
+            const double a[4] = {lo ? a0[0] : a1[0], lo ? a0[1] : a1[1], lo ? a0[2] : a1[2],
+                                 lo ? a0[3] : a1[3]};
+            dmma(acc[f], a, b);
+          }
+        }
+        if (kk == 0) mid_stage(it);
+      }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int f = 0; f < F; ++f)
+      if (f < d.count) store(f < d.split ? d.r0 : d.r1, (bo[f] - g) / 8, acc[f]);
+    return;
+  }
+  // off the diagonal: row tile `warp`, all column tiles, in groups of 4
+  double acc[BN / 8][4];
+#pragma unroll
+  for (int j = 0; j < BN / 8; ++j)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[j][c] = 0.0;
   for (int it = 0; it < nstage; ++it) {
-    cp_async_wait<NS - 2>();
-    __syncthreads();
-    if (it + NS - 1 < nstage) load_stage(it + NS - 1);
-    cp_async_commit();
+    begin_stage(it);
     const int slot = it % NS;
     const double(*bt)[LDA] = sm.b[slot];
     const double *w = sm.w[slot];
-    stage_mma(sm.a[slot], wrow, g, q,
-              [&](int nt, int kk, double(&b)[2]) {
-                const int c = wcol + nt * 8 + g;
-                b[0] = bt[c][kk + q] * w[kk + q];
-                b[1] = bt[c][kk + q + 4] * w[kk + q + 4];
-              },
-              acc);
+#pragma unroll
+    for (int kk = 0; kk < BK; kk += 8) {
+      const double w0 = w[kk + q], w1 = w[kk + q + 4];
+      const double *x = &sm.a[slot][16 * warp + g][kk + q];
+      const double a[4] = {x[0], x[8 * LDA], x[4], x[8 * LDA + 4]};
+#pragma unroll
+      for (int j4 = 0; j4 < BN / 8; j4 += 4) {
+        if (j4 >= ncol) continue;                  // uniform
+#pragma unroll
+        for (int j = j4; j < j4 + 4; ++j) {
+          const double b[2] = {bt[8 * j + g][kk + q] * w0, bt[8 * j + g][kk + q + 4] * w1};
+          dmma(acc[j], a, b);
+        }
+      }
+      if (kk == 0) mid_stage(it);
+    }
   }
   cp_async_wait<0>();
-  const int ntile = nblk * (nblk + 1) / 2;
-  double *out = work + ((long)ck * ntile + tile_index) * (BM * BN);
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int r = wrow + mt * 16 + g, c = wcol + nt * 8 + 2 * q;
-      *reinterpret_cast<double2 *>(out + r * BN + c) = make_double2(acc[mt][nt][0], acc[mt][nt][1]);
-      *reinterpret_cast<double2 *>(out + (r + 8) * BN + c) =
-          make_double2(acc[mt][nt][2], acc[mt][nt][3]);
-    }
+  for (int j = 0; j < BN / 8; ++j)
+    if (j < ncol) store(warp, j, acc[j]);
 }
 
 __global__ void __launch_bounds__(NT, 1)
 quadrature_kernel(int n, int npoint_pad, const double *__restrict__ phi,
                   const double *__restrict__ phib, long ld,
-                  const double *__restrict__ wv, int nblk, int chunk,
+                  const double *__restrict__ wv, const QuadPlan plan,
                   double *__restrict__ work, const int *__restrict__ blocks) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   QuadSmem &sm = *reinterpret_cast<QuadSmem *>(smem_raw);
-  quadrature_block(sm, n, npoint_pad, phi, phib, ld, wv, nblk, chunk, work, blocks,
-                   blockIdx.x, blockIdx.y);
+  quadrature_block(sm, n, npoint_pad, phi, phib, ld, wv, plan, work, blocks, blockIdx.x);
 }
 
-__global__ void quadrature_reduce_kernel(int n, int nblk, int nchunk,
-                                         const double *__restrict__ work,
-                                         double *__restrict__ F) {
-  const int ntile = nblk * (nblk + 1) / 2;
-  const long total = (long)ntile * BM * BN;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
-       e += (long)gridDim.x * blockDim.x) {
-    const int tile = (int)(e / (BM * BN));
-    const int m = (int)(e % (BM * BN)) / BN, c = (int)(e % BN);
-    int mb = 0, rem = tile;
-    while (rem >= nblk - mb) {
-      rem -= nblk - mb;
-      ++mb;
+// Entries of all partial sums, in groups of 32 (a CTA of the reduction each).
+__host__ __device__ inline long quad_entry_groups(int n) {
+  if (n <= kSmallN) return 4L * small_frags(small_tiles(n));
+  const long nblk = (n + BM - 1) / BM;
+  return nblk * (nblk + 1) / 2 * (BM * BN / 32);
+}
+
+// Adds the chunks' partial sums in a fixed order and writes both triangles of
+// F; a CTA owns 32 consecutive entries.  One thread per entry over all chunks
+// took 54 us for H2O (592 dependent loads) and 35 us for C8H18.
+// n <= 64: chunks in order, staged through shared memory by all 8 warps
+// kRedRows at a time while warp 0 adds the rows staged before them.
+// n > 64: 8 warps take chunks w, w + 8, ..., then the warps in order.
+constexpr int kRedRows = 64;
+struct ReduceSmem {
+  double row[2][kRedRows][32];
+};
+__device__ __forceinline__ void quadrature_reduce_block(ReduceSmem &sm, int n,
+                                                        const QuadPlan &plan,
+                                                        const double *__restrict__ work,
+                                                        double *__restrict__ F, long bx) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int mu, nu, nchunk;
+  long stride;                          // doubles from one chunk's entry to the next's
+  const double *w = work + lane;        // the entry in chunk 0
+  if (n <= kSmallN) {
+    const int rt = small_tiles(n), c = (int)(bx & 3);
+    int f = (int)(bx >> 2), i = 0;
+    while (f >= 2 * (rt - i)) f -= 2 * (rt - i++);
+    mu = 16 * i + (lane >> 2) + 8 * (c >> 1);
+    nu = 8 * (2 * i + f) + 2 * (lane & 3) + (c & 1);
+    nchunk = plan.nch[0];
+    stride = 128L * small_frags(rt);
+    w += bx * 32;
+  } else {
+    constexpr int G = BM * BN / 32;     // groups per tile
+    int tile = (int)(bx / G), cls = 0;
+    const int e = (int)(bx % G) * 32 + lane;
+    while (tile >= plan.ntile[cls]) tile -= plan.ntile[cls++];
+    int mb, nb;
+    quad_tile(cls, tile, (n + BM - 1) / BM, mb, nb);
+    mu = mb * BM + e / BN;
+    nu = nb * BN + e % BN;
+    nchunk = plan.nch[cls];
+    stride = (long)plan.ntile[cls] * BM * BN;
+    w += (long)(plan.first[cls] + tile) * BM * BN + (bx % G) * 32;
+  }
+  const bool live = mu <= nu && nu < n;
+  if (!__syncthreads_or(live)) return;
+  double s = 0.0;
+  if (n <= kSmallN) {
+    constexpr int PER = kRedRows / kWarps;
+    double r[PER];
+    auto fetch = [&](int k0) {  // rows warp, warp + 8, ... of a round
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int k = k0 + warp + kWarps * i;
+        r[i] = k < nchunk ? __ldg(w + k * stride) : 0.0;
+      }
+    };
+    fetch(0);
+    for (int k0 = 0, buf = 0; k0 < nchunk; k0 += kRedRows, buf ^= 1) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i) sm.row[buf][warp + kWarps * i][lane] = r[i];
+      __syncthreads();
+      if (k0 + kRedRows < nchunk) fetch(k0 + kRedRows);
+      if (warp == 0) {
+#pragma unroll 16
+        for (int i = 0; i < kRedRows; ++i) s += sm.row[buf][i][lane];
+      }
     }
-    const int nb = mb + rem;
-    const int mu = mb * BM + m, nu = nb * BN + c;
-    if (mu >= n || nu >= n || mu > nu) continue;
-    double s = 0.0;
-    for (int k = 0; k < nchunk; ++k) s += work[((long)k * ntile + tile) * (BM * BN) + m * BN + c];
+  } else {
+    if (live) {
+#pragma unroll 4
+      for (int k = warp; k < nchunk; k += kWarps) s += __ldg(w + k * stride);
+    }
+    sm.row[0][warp][lane] = s;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int k = 1; k < kWarps; ++k) s += sm.row[0][k][lane];
+    }
+  }
+  if (warp == 0 && live) {
     F[(long)mu * n + nu] = s;
     F[(long)nu * n + mu] = s;
   }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(NT)
+quadrature_reduce_kernel(int n, const QuadPlan plan, const double *__restrict__ work,
+                         double *__restrict__ F) {
+  __shared__ ReduceSmem sm;
+  quadrature_reduce_block(sm, n, plan, work, F, blockIdx.x);
 }
 
 __global__ void combine_weights_kernel(int npoint, const double *__restrict__ wb,
@@ -417,20 +799,71 @@ __global__ void combine_weights_kernel(int npoint, const double *__restrict__ wb
   wv[p] = wb[p] * w[p] * pot;
 }
 
-inline int quad_chunks(int n, int npoint_pad, int *chunk_out) {
-  const int nblk = (n + BM - 1) / BM;
-  const int ntile = nblk * (nblk + 1) / 2;
-  // one CTA per SM at these register counts: aim for ~4 full waves over the
-  // 148 SMs so the last wave is (nearly) full
-  int nchunk = (4 * 148) / ntile;
-  if (nchunk < 1) nchunk = 1;
-  int chunk = (npoint_pad + nchunk - 1) / nchunk;
-  chunk = ((chunk + BK - 1) / BK) * BK;
-  if (chunk < BK) chunk = BK;
-  nchunk = (npoint_pad + chunk - 1) / chunk;
-  *chunk_out = chunk;
-  return nchunk;
+// Cost of a stage of one tile: DMMA instructions per k8 step of the busiest
+// sub-partition (warps w and w + 4), plus the stage's fixed part (barrier and
+// copies, about 4 of them).
+inline int quad_tile_cost(int n, int nblk, int cls) {
+  const bool ragged = cls == 1 || cls == 3;
+  const int cols = ragged ? n - (nblk - 1) * BN : BN;
+  const int C = (cols + 7) / 8, R = (cols + 15) / 16;
+  const int groups4 = (C + 3) / 4 * 4, frags3 = (C - R + 1 + 2) / 3 * 3;
+  return 4 + (cls < 2 ? 2 * groups4 : (R > 4 ? 2 : 1) * frags3);
 }
+
+// The split for at most `slots` partial tiles (n > 64) or chunks (n <= 64).
+// *bound (optional) receives the most slots that any range of at most npad
+// points uses: a shorter range can be cut into more chunks (chunk lengths are
+// rounded up to 16 points), up to one per 16 points and the counts below.
+QuadPlan quad_plan_slots(int n, int npad, int slots, long *bound = nullptr) {
+  QuadPlan p = {};
+  if (bound) *bound = 0;
+  auto split = [&](int c) {  // chunk length and count for at most nch[c] chunks
+    if (bound) *bound += (long)p.ntile[c] * std::max(std::min(p.nch[c], npad / BK), 1);
+    int chunk = (npad + p.nch[c] - 1) / p.nch[c];
+    chunk = std::max((chunk + BK - 1) / BK * BK, BK);
+    p.chunk[c] = chunk;
+    p.nch[c] = (npad + chunk - 1) / chunk;
+  };
+  if (n <= kSmallN) {
+    p.ntile[0] = 1;
+    p.nch[0] = slots;
+    split(0);
+    for (int c = 1; c < 5; ++c) p.first[c] = p.nch[0];
+    return p;
+  }
+  const int nblk = (n + BM - 1) / BM;
+  p.ntile[0] = (nblk - 1) * (nblk - 2) / 2;
+  p.ntile[1] = nblk - 1;
+  p.ntile[2] = nblk - 1;
+  p.ntile[3] = 1;
+  long total = 0;
+  int cost[4];
+  for (int c = 0; c < 4; ++c) {
+    cost[c] = quad_tile_cost(n, nblk, c);
+    total += (long)cost[c] * p.ntile[c];
+  }
+  // chunks in proportion to the cost, so that all CTAs take about as long
+  for (int s = slots;; --s) {
+    long used = 0;
+    bool single = true;
+    for (int c = 0; c < 4; ++c) {
+      p.nch[c] = (int)std::max<long>((long)s * cost[c] / total, 1);
+      used += (long)p.nch[c] * p.ntile[c];
+      single = single && p.nch[c] == 1;
+    }
+    if (used <= slots || single) break;
+  }
+  for (int c = 0; c < 4; ++c) {
+    split(c);
+    p.first[c + 1] = p.first[c] + p.nch[c] * p.ntile[c];
+  }
+  return p;
+}
+
+// Slots: n <= 64 (a warp per chunk) four warps per SM; n > 64 (a CTA per slot,
+// one CTA per SM at these register counts) two full waves over the 148 SMs for
+// a single tile, four otherwise.
+inline int quad_default_slots(int n) { return n > kSmallN && n <= BM ? 2 * 148 : 4 * 148; }
 
 inline int pad_points(int npoint) { return ((npoint + BN - 1) / BN) * BN; }
 
@@ -450,6 +883,17 @@ cudaError_t launch_density_f64(int n, int npoint, const double *phi, long ld,
     blocks = ngroup;
     if (blocks == 0) return cudaSuccess;
   }
+  if (n <= kSmallN) {
+    // a CTA takes several groups once there are four CTAs per SM
+    const int grid = std::min(blocks, 148 * 4);
+    switch (small_tiles(n)) {
+      case 1: density_small_kernel<1><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep); break;
+      case 2: density_small_kernel<2><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep); break;
+      case 3: density_small_kernel<3><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep); break;
+      default: density_small_kernel<4><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep);
+    }
+    return cudaGetLastError();
+  }
   // 16-byte copies of D rows need n even and a 16-byte aligned D
   const bool vec = n % 2 == 0 && reinterpret_cast<uintptr_t>(D) % 16 == 0;
   auto kern = vec ? density_kernel<true> : density_kernel<false>;
@@ -460,24 +904,41 @@ cudaError_t launch_density_f64(int n, int npoint, const double *phi, long ld,
   return cudaGetLastError();
 }
 
-// the split-K quadrature kernel with its dynamic shared memory
-cudaError_t quadrature_launch(dim3 grid, int n, int npad, const double *phi, const double *phib,
-                              long ld, const double *wv, int nblk, int chunk, double *work,
-                              cudaStream_t s, const int *blocks = nullptr) {
-  cudaError_t e = cudaFuncSetAttribute(quadrature_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)kQuadSmem);
-  if (e != cudaSuccess) return e;
-  quadrature_kernel<<<grid, NT, kQuadSmem, s>>>(n, npad, phi, phib, ld, wv, nblk, chunk, work,
-                                                blocks);
+QuadPlan quad_plan(int n, int npad) { return quad_plan_slots(n, npad, quad_default_slots(n)); }
+
+int quad_plan_items(int n, const QuadPlan &p) {
+  return n <= kSmallN ? (p.nch[0] + kWarps - 1) / kWarps : p.first[4];
+}
+
+// the split-K quadrature and the sum of its chunks
+cudaError_t quadrature_launch(const QuadPlan &plan, int n, int npad, const double *phi,
+                              const double *phib, long ld, const double *wv, double *work,
+                              double *F, cudaStream_t s, const int *blocks = nullptr) {
+  cudaError_t e;
+  if (n <= kSmallN) {
+    auto kern = small_tiles(n) == 1   ? quadrature_small_kernel<1>
+                : small_tiles(n) == 2 ? quadrature_small_kernel<2>
+                : small_tiles(n) == 3 ? quadrature_small_kernel<3>
+                                      : quadrature_small_kernel<4>;
+    // four warps per CTA: the chunks spread over all SMs
+    kern<<<(plan.nch[0] + 3) / 4, 128, 0, s>>>(n, npad, phi, phib, ld, wv, plan.chunk[0], work,
+                                              blocks);
+  } else {
+    e = cudaFuncSetAttribute(quadrature_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kQuadSmem);
+    if (e != cudaSuccess) return e;
+    quadrature_kernel<<<plan.first[4], NT, kQuadSmem, s>>>(n, npad, phi, phib, ld, wv, plan, work,
+                                                          blocks);
+  }
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  quadrature_reduce_kernel<<<(unsigned)quad_entry_groups(n), NT, 0, s>>>(n, plan, work, F);
   return cudaGetLastError();
 }
 
 size_t quadrature_workspace_bytes(int n, int npoint) {
-  int chunk;
-  const int nchunk = quad_chunks(n, pad_points(npoint), &chunk);
-  const int nblk = (n + BM - 1) / BM;
-  return (size_t)nchunk * (nblk * (nblk + 1) / 2) * BM * BN * sizeof(double);
+  long slots = 0;
+  quad_plan_slots(n, pad_points(npoint), quad_default_slots(n), &slots);
+  return slots * (n <= kSmallN ? 128 * small_frags(small_tiles(n)) : BM * BN) * sizeof(double);
 }
 
 cudaError_t launch_quadrature_f64(int n, int npoint, const double *phi, long ld,
@@ -486,32 +947,10 @@ cudaError_t launch_quadrature_f64(int n, int npoint, const double *phi, long ld,
                                   int nblock) {
   if (!phib) phib = phi;
   if (n <= 0) return cudaSuccess;
-  // screened: the K range is the listed 16-point blocks; its chunk count is
-  // capped at the workspace's (sized for every point), see quadrature_chunking
+  // screened: the K range is the listed 16-point blocks
   const int npad = blocks ? nblock * BK : pad_points(npoint);
   if (npad == 0) return cudaMemsetAsync(F, 0, (size_t)n * n * sizeof(double), s);
-  int chunk;
-  const int nchunk = quadrature_chunking(n, npad, &chunk, pad_points(npoint));
-  const int nblk = (n + BM - 1) / BM;
-  const int ntile = nblk * (nblk + 1) / 2;
-  dim3 grid(ntile, nchunk);
-  cudaError_t e = quadrature_launch(grid, n, npad, phi, phib, ld, wv, nblk, chunk, work, s,
-                                    blocks);
-  if (e != cudaSuccess) return e;
-  const long total = (long)ntile * BM * BN;
-  const int rblocks = (int)std::min<long>((total + 255) / 256, 148 * 16);
-  quadrature_reduce_kernel<<<rblocks, 256, 0, s>>>(n, nblk, nchunk, work, F);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_quadrature_reduce(int n, int nchunk, const double *work, double *F,
-                                     cudaStream_t s) {
-  const int nblk = (n + BM - 1) / BM;
-  const int ntile = nblk * (nblk + 1) / 2;
-  const long total = (long)ntile * BM * BN;
-  const int rblocks = (int)std::min<long>((total + 255) / 256, 148 * 16);
-  quadrature_reduce_kernel<<<rblocks, 256, 0, s>>>(n, nblk, nchunk, work, F);
-  return cudaGetLastError();
+  return quadrature_launch(quad_plan(n, npad), n, npad, phi, phib, ld, wv, work, F, s, blocks);
 }
 
 // -------------------------------------------------------------- batches
@@ -562,6 +1001,11 @@ density_batch_kernel(const DensBatchArg *__restrict__ args, BatchQueue q) {
     if (w < 0) break;
     const int4 it = q.items[w];
     const DensBatchArg a = args[it.x];
+    if (a.n <= kSmallN) {  // group it.y alone
+      density_small_any(a.n, a.npoint, a.phi, a.ld, a.D, a.rho, nullptr, it.y + 1, it.y, 1,
+                        a.keep);
+      continue;
+    }
     if (a.vecD)
       density_block<true>(sm, a.n, a.npoint, a.phi, a.ld, a.D, a.rho, it.y * BN, a.keep);
     else
@@ -579,33 +1023,28 @@ quadrature_batch_kernel(const QuadBatchArg *__restrict__ args, BatchQueue q) {
     if (w < 0) break;
     const int4 it = q.items[w];
     const QuadBatchArg a = args[it.x];
-    quadrature_block(sm, a.n, a.npad, a.phi, a.phi, a.ld, a.wv, a.nblk, a.chunk, a.work,
-                     a.blocks, it.y, it.z);
+    if (a.n <= kSmallN) {  // chunks 8 it.y .. 8 it.y + 7, one per warp
+      const int ck = kWarps * it.y + (threadIdx.x >> 5), chunk = a.plan.chunk[0];
+      switch (small_tiles(a.n)) {
+        case 1: quadrature_small_chunk<1, true>(a.n, a.npad, a.phi, a.phi, a.ld, a.wv, chunk, a.work, a.blocks, ck); break;
+        case 2: quadrature_small_chunk<2, true>(a.n, a.npad, a.phi, a.phi, a.ld, a.wv, chunk, a.work, a.blocks, ck); break;
+        case 3: quadrature_small_chunk<3, true>(a.n, a.npad, a.phi, a.phi, a.ld, a.wv, chunk, a.work, a.blocks, ck); break;
+        default: quadrature_small_chunk<4, true>(a.n, a.npad, a.phi, a.phi, a.ld, a.wv, chunk, a.work, a.blocks, ck);
+      }
+      continue;
+    }
+    quadrature_block(sm, a.n, a.npad, a.phi, a.phi, a.ld, a.wv, a.plan, a.work, a.blocks, it.y);
   }
 }
 
 // F of every molecule from its chunk partials (blockIdx.y = molecule)
-__global__ void quadrature_reduce_batch_kernel(const QuadBatchArg *__restrict__ args) {
+__global__ void __launch_bounds__(NT)
+quadrature_reduce_batch_kernel(const QuadBatchArg *__restrict__ args) {
+  __shared__ ReduceSmem sm;
   const QuadBatchArg a = args[blockIdx.y];
-  const int ntile = a.nblk * (a.nblk + 1) / 2;
-  const long total = (long)ntile * BM * BN;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
-       e += (long)gridDim.x * blockDim.x) {
-    const int tile = (int)(e / (BM * BN));
-    const int m = (int)(e % (BM * BN)) / BN, c = (int)(e % BN);
-    int mb = 0, rem = tile;
-    while (rem >= a.nblk - mb) {
-      rem -= a.nblk - mb;
-      ++mb;
-    }
-    const int nb = mb + rem;
-    const int mu = mb * BM + m, nu = nb * BN + c;
-    if (mu >= a.n || nu >= a.n || mu > nu) continue;
-    double s = 0.0;
-    for (int k = 0; k < a.nchunk; ++k) s += a.work[((long)k * ntile + tile) * (BM * BN) + m * BN + c];
-    a.F[(long)mu * a.n + nu] = s;
-    a.F[(long)nu * a.n + mu] = s;
-  }
+  const long nb = quad_entry_groups(a.n);
+  for (long b = blockIdx.x; b < nb; b += gridDim.x)
+    quadrature_reduce_block(sm, a.n, a.plan, a.work, a.F, b);
 }
 
 // wv of every molecule (blockIdx.y), zero padded to its npad points
@@ -616,25 +1055,6 @@ __global__ void combine_weights_batch_kernel(const WeightBatchArg *__restrict__ 
 }
 
 }  // namespace
-
-// Chunking of a K range of npad points when the workspace was sized for a
-// grid of pad_full points (npad <= pad_full): quad_chunks is not monotone in
-// the range (a shorter range below a chunk-size step gets more, shorter
-// chunks), so the chunk count is capped at the full grid's and the chunks
-// lengthened to fit.
-int quadrature_chunking(int n, int npad, int *chunk, int pad_full) {
-  int c = 0;
-  int nchunk = quad_chunks(n, npad, &c);
-  int cf = 0;
-  const int cap = quad_chunks(n, pad_full > npad ? pad_full : npad, &cf);
-  if (nchunk > cap) {
-    c = (npad + cap - 1) / cap;
-    c = ((c + BK - 1) / BK) * BK;
-    nchunk = (npad + c - 1) / c;
-  }
-  *chunk = c;
-  return nchunk;
-}
 
 cudaError_t launch_density_batch(const DensBatchArg *args, const BatchQueue &q, int grid,
                                  cudaStream_t s) {
@@ -660,7 +1080,7 @@ cudaError_t launch_quadrature_batch(const QuadBatchArg *args, const BatchQueue &
 
 cudaError_t launch_quadrature_reduce_batch(const QuadBatchArg *args, int nmol, cudaStream_t s) {
   if (nmol == 0) return cudaSuccess;
-  quadrature_reduce_batch_kernel<<<dim3(148 * 2, nmol), 256, 0, s>>>(args);
+  quadrature_reduce_batch_kernel<<<dim3(148 * 4, nmol), NT, 0, s>>>(args);
   return cudaGetLastError();
 }
 
@@ -797,9 +1217,8 @@ int napmo_gpu_quadrature_noalloc(int n, int npoint, const double *phi, const dou
   const int npad = pad_points(npoint);
   if (ld < npad || ld % 2 != 0)
     return set_error(kInvalidArgument, "ld must be even and >= npoint rounded up to 128");
-  const int nblk = (n + BM - 1) / BM;
-  const int ntile = nblk * (nblk + 1) / 2;
-  const size_t per_chunk = (size_t)ntile * BM * BN;
+  const long nblk = (n + BM - 1) / BM;
+  const size_t per_chunk = (size_t)(nblk * (nblk + 1) / 2) * BM * BN;
   if (per_chunk > kNoAllocScratchDoubles)
     return set_error(kInvalidArgument,
                      "napmo_gpu_quadrature_noalloc: n = " + std::to_string(n) +
@@ -813,24 +1232,14 @@ int napmo_gpu_quadrature_noalloc(int n, int npoint, const double *phi, const dou
   double *scratch = nullptr;
   int st = scratch_address(&scratch);
   if (st != kOk) return st;
-  // as many chunks as the launch policy wants, capped by the fixed array
-  int chunk;
-  int nchunk = quad_chunks(n, npad, &chunk);
-  const int cap = (int)(kNoAllocScratchDoubles / per_chunk);
-  if (nchunk > cap) {
-    chunk = (npad + cap - 1) / cap;
-    chunk = ((chunk + BK - 1) / BK) * BK;
-    nchunk = (npad + chunk - 1) / chunk;
-  }
-  dim3 grid(ntile, nchunk);
-  cudaError_t e = quadrature_launch(grid, n, npad, phi, psi ? psi : phi, ld, wv, nblk, chunk,
-                                    scratch, s);
+  // the launch policy's split, capped by the fixed array
+  int slots = quad_default_slots(n);
+  if (n > kSmallN) slots = std::min(slots, (int)(kNoAllocScratchDoubles / (BM * BN)));
+  static_assert(4 * 148 * 128 * small_frags(kSmallN / 16) <= (int)kNoAllocScratchDoubles,
+                "the small molecules' partial sums fit the fixed array");
+  const cudaError_t e = quadrature_launch(quad_plan_slots(n, npad, slots), n, npad, phi,
+                                          psi ? psi : phi, ld, wv, scratch, F, s);
   if (e != cudaSuccess) return set_error(kCudaError, std::string("quadrature: ") + cudaGetErrorString(e));
-  const long total = (long)ntile * BM * BN;
-  const int rblocks = (int)std::min<long>((total + 255) / 256, 148 * 16);
-  quadrature_reduce_kernel<<<rblocks, 256, 0, s>>>(n, nblk, nchunk, scratch, F);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return set_error(kCudaError, std::string("quadrature reduce: ") + cudaGetErrorString(e));
   return kOk;
 }
 
