@@ -42,7 +42,7 @@ struct PoissonPlan {
   std::vector<PoissonAtom> h_atoms;
   DevBuf<PoissonAtom> atoms;
   DevBuf<int> mol_atom_off, mol_point_off, sys_atom, sys_l;
-  DevBuf<double> rad, ytab, proj, spl, amp, raw_y, raw_dt, lu, lmul;
+  DevBuf<double> rad, ytab, proj, spl, rows, amp, raw_y, raw_dt, lu, lmul;
   DevBuf<int> lpiv;
   DevBuf<double> rscr;  // radial-solve scratch of one solve
   DevBuf<double> pg;    // projection scratch of one solve (rho wb w per point)
@@ -105,7 +105,7 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
   std::vector<double> rad, ytab;
   std::map<std::pair<int, int>, int> ykey;  // (atom-rule id via nang,lmax) -> offset
   std::vector<int> sys_atom, sys_l;
-  long proj = 0, spl = 0, amp = 0, raw = 0, pairs = 0, scr = 0, npts = 0;
+  long proj = 0, spl = 0, rows = 0, amp = 0, raw = 0, pairs = 0, scr = 0, npts = 0;
   int buckets = 0;
   std::vector<int> atom_mol(natom, 0);
   for (int m = 0; m + 1 < (int)mol_atom_off.size(); ++m)
@@ -162,6 +162,8 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
     proj += (long)n * lsize;
     A.spl_off = (int)spl;
     spl += (long)(n - 1) * lsize * 4;
+    A.rows_off = rows;
+    rows += (long)(n - 1) * (long)eval_rows_doubles(lmax);
     A.amp_off = (int)amp;
     amp += (long)lsize * 2;
     A.raw_off = (int)raw;
@@ -196,6 +198,7 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
   NAPMO_TRY_CUDA(plan->ytab.upload(ytab, s), "upload harmonics");
   NAPMO_TRY_CUDA(plan->proj.alloc(proj), "alloc");
   NAPMO_TRY_CUDA(plan->spl.alloc(spl), "alloc");
+  NAPMO_TRY_CUDA(plan->rows.alloc(rows), "alloc");
   NAPMO_TRY_CUDA(plan->amp.alloc(amp), "alloc");
   NAPMO_TRY_CUDA(plan->raw_y.alloc(raw), "alloc");
   NAPMO_TRY_CUDA(plan->raw_dt.alloc(raw), "alloc");
@@ -210,6 +213,7 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
   d.ytab = plan->ytab.p;
   d.proj = plan->proj.p;
   d.spl = plan->spl.p;
+  d.rows = plan->rows.p;
   d.amp = plan->amp.p;
   d.raw_y = plan->raw_y.p;
   d.raw_dt = plan->raw_dt.p;
@@ -228,12 +232,13 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
   return kOk;
 }
 
-// Pairs per evaluation item (CTA of chunk / 2 threads): a larger item shares
-// one staging of its interval's coefficients among more pairs, but leaves
-// fewer CTAs and, at 256 threads and 76 registers, fewer resident warps.  On B200,
-// 512-pair items made the C20H42 100x302 evaluation 5 % faster (about 15,000
-// pairs per interior bucket) and the H2O 50x110 and HCN 100x302 SCFs (300
-// and 900 pairs) slower than 128-pair items.
+// Pairs per evaluation item (CTA of chunk / 4 threads): a larger item shares
+// one copy of its interval's coefficients among more pairs, but the last item
+// of a bucket is emptier and the CTAs are fewer.  On B200 the C12H26 100x302
+// evaluation (11,600 pairs per interior bucket) took 3.54 ms with 512-pair
+// items (1024: 3.72), 35 solves of HCN 100x302 (900 pairs) 850 us with 128
+// (256: 910, 512: 962), 75 of H2O 50x110 (330 pairs) 204 us (256: 236,
+// 512: 311); at C5H12 75x194 (3,300 pairs) they differ by 4 %.
 static int eval_chunk_for(const std::vector<int> &count, const std::vector<PoissonAtom> &ha) {
   long pairs = 0, buckets = 0;
   for (const PoissonAtom &a : ha)
@@ -537,7 +542,7 @@ int run_poisson_many(BeckeGrid *g, PoissonPlan *p, int k, const double *rho_dev,
   int st = select_pair_lists(p, g, keep, key, s);
   if (st) return st;
   const PoissonDev &d = p->d;
-  const size_t nd = p->proj.n + p->spl.n + p->amp.n + p->pair_v.n + p->rscr.n + p->pg.n;
+  const size_t nd = p->proj.n + p->spl.n + p->rows.n + p->amp.n + p->pair_v.n + p->rscr.n + p->pg.n;
   const size_t per = nd * sizeof(double) + p->lcut.n * sizeof(int);
   // grid limits: the projection and truncation launches use natom x B blocks
   // in y/z, the radial one B in y
@@ -559,12 +564,14 @@ int run_poisson_many(BeckeGrid *g, PoissonPlan *p, int k, const double *rho_dev,
   P.batch_ld = ld;
   P.proj_stride = (long)p->proj.n;
   P.spl_stride = (long)p->spl.n;
+  P.rows_stride = (long)p->rows.n;
   P.amp_stride = (long)p->amp.n;
   P.pairv_stride = (long)p->pair_v.n;
   P.lcut_stride = (long)p->lcut.n;
   P.rscr_stride = (long)p->rscr.n;
   double *ws = (double *)p->batch_ws.p;
-  P.proj = ws;
+  P.rows = ws;  // first: its 16-byte copies need the allocation's alignment
+  P.proj = P.rows + P.rows_stride * B;
   P.spl = P.proj + P.proj_stride * B;
   P.amp = P.spl + P.spl_stride * B;
   P.pair_v = P.amp + P.amp_stride * B;

@@ -42,11 +42,16 @@ __constant__ double c_shnorm[(kMaxLmax + 1) * (kMaxLmax + 1)];  // [l][m]
 // A_lm = a_lm gamma_(l-1) / gamma_l: one product and one FMA per step.  The
 // coefficients multiplying q_l are scaled by gamma_lm when staged.
 __constant__ double c_rec_a[(kMaxLmax + 1) * (kMaxLmax + 1)];      // A_lm at [l][m]
-__constant__ double c_rec_gamma[(kMaxLmax + 1) * (kMaxLmax + 1)];  // gamma at [lm]
 __constant__ double c_rec_start[kMaxLmax + 1];
-// global copy of c_rec_gamma for staging loops whose lanes read different
-// entries (constant memory serves one address at a time)
+// gamma at [lm], for staging loops whose lanes read different entries (constant
+// memory serves one address at a time)
 __device__ double g_rec_gamma[(kMaxLmax + 1) * (kMaxLmax + 1)];
+// Staging factors of the interior evaluation (interior_values): g_eval_alpha
+// at [lm] is gamma_lm for even m and the norm of S_lm over its Gegenbauer
+// polynomial for odd m; g_eval_beta at [l][m], m even, is (2l + 1) gamma_lm /
+// norm_lm.
+__device__ double g_eval_alpha[(kMaxLmax + 1) * (kMaxLmax + 1)];
+__device__ double g_eval_beta[(kMaxLmax + 1) * (kMaxLmax + 1)];
 // Finite-difference weights of the radial second derivative (integers over
 // common denominators, host deriv2_stencils()): [0, 28) first derivative at
 // the four edge nodes (7 weights each), [28, 56) second derivative, [56, 65)
@@ -1044,59 +1049,187 @@ __global__ void pair_scatter_kernel(PoissonDev P, const double *__restrict__ gx,
 
 // One CTA per EvalItem: the coefficient block of the item's spline interval
 // (or the tail amplitudes) is staged in shared memory once and every thread
-// evaluates one pair:
+// evaluates four pairs:
 //   v_pair = sum_k u^k sum_lm S_lm(r_hat) c_k,lm        (interval)
 //   v_pair = sum_l g_l(d) sum_m S_lm(r_hat) a_lm         (tails, g = d^l or
 //                                                         d^-(l+1))
 // with S_lm(r_hat) = S_lm(p - A) / d^l, so the 1/d^l of the reference is folded
 // into the unit vector.  The result goes to the pair's own slot of pair_v.
-// Potentials of NP (atom, point) pairs of one bucket from the shared
-// coefficients cf (each coefficient load serves all NP pairs): REGION 0
-// inside the atom's radial grid (cubic spline in the interval coordinate u),
-// 1 below its first point (amplitudes x d^l), 2 beyond its last (amplitudes
-// x d^-(l+1)).
-template <int LMAX, int REGION, int NP>
-__device__ __forceinline__ void pair_values(const double *cf, int lmaxA, const double *x,
-                                            const double *y, const double *z, const double *d,
-                                            const double *inv, const double *u, double *v) {
-  double a0[NP], a1[NP], a2[NP], a3[NP], gstep[NP], cm[NP], sm[NP], gm[NP];
+//
+// Normalised solid harmonics of the unit vector: S_l0 = q_l^0, S_lm (cos, sin)
+// = q_l^m Re/Im (x + iy)^m at lm = l^2 + 2m - 1, l^2 + 2m (solid_harmonics.h),
+// q_l^m = nrm_lm Pi_l^m with Pi_m^m = (2m-1)!!, Pi_(m+1)^m = (2m+1) z Pi_m^m,
+// Pi_l^m = ((2l-1) z Pi_(l-1)^m - (l+m-1) Pi_(l-2)^m) / (l-m) (|u| = 1); the
+// recursion runs on q~ = q / gamma (c_rec_a, c_rec_start).
+//
+// Interior pairs (NP of one spline interval; each coefficient load serves all
+// of them).  The FP64 pipe bounds this function, so what is not a product with
+// a coefficient is kept off the (l, m) level:
+//  - columns m0 and m0 + 1 (m0 even) share one recursion.  Pi_l^m is (2m-1)!!
+//    times the Gegenbauer polynomial C_(l-m)^(m+1/2), and C_n^(s+1) = sum_k
+//    (n - 2k + s) / s C_(n-2k)^s, so a combination of column m0 + 1 is one of
+//    column m0 with the suffix sums of its coefficients (stage_interior forms
+//    them, once per CTA).  Sharing more columns would save little more and
+//    lose digits: the sums of |terms| grow to 3 times the result for two
+//    columns, 65 for four, 3500 for all (lmax 20).
+//  - the sum over l of one column is complete before it meets cos/sin(m phi),
+//  - each coefficient is the cubic's value at u (3 FMAs), then one FMA with q~.
+// Per pair at lmax 14: 1100 FP64 operations, 900 of them the cubics and their
+// sums; a recursion per column with the products q cos, q sin and four sums
+// (over k) took 1380.  Four pairs per thread halve the shared-memory reads of
+// two (their pipe was 68 % busy), the cubics of two series run side by side,
+// and the loop over l stays rolled (unrolled to lmax 20 it outgrew the
+// instruction cache).  Interior evaluation, before -> now: C12H26 100 x 302
+// 4.11 -> 3.55 ms, C5H12 75 x 194 288 -> 248 us, HCN 100 x 302 x 35 solves
+// 1.05 -> 0.85 ms.
+constexpr int kEvalRow = 16;  // doubles of a row: (cos, sin of m0; of m0 + 1) x 4
+__host__ __device__ constexpr int eval_family(int lmax, int f) {  // first row of m0 = 2f
+  return f * (lmax + 1) - f * (f - 1);
+}
+__host__ __device__ constexpr int eval_rows(int lmax) { return eval_family(lmax, lmax / 2 + 1); }
+
+// One family: columns m0 and m0 + 1, rows n < nodd of both and row nodd of m0
+// alone (m0 + 1 has its last term one row before).
+template <int NP, bool SIN>
+__device__ __forceinline__ void family_sums(const double *row, int nodd, const double *rec,
+                                            double start, const double *z, const double *u,
+                                            double *ec, double *es, double *oc, double *os) {
+  double b[NP], bp[NP];
+  // s[g] += (cubic of the four doubles at c + 4 g)(u) b, the G cubics level by
+  // level: G x NP independent products in flight
+  auto add = [&](const double *c, auto &...s) {
+    constexpr int G = sizeof...(s);
+    double *const sp[G] = {s...};
+    double2 lo[G], hi[G];
+    double t[G][NP];
+#pragma unroll
+    for (int g = 0; g < G; ++g) hi[g] = *reinterpret_cast<const double2 *>(c + 4 * g + 2);
+#pragma unroll
+    for (int g = 0; g < G; ++g) lo[g] = *reinterpret_cast<const double2 *>(c + 4 * g);
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) t[g][j] = fma(hi[g].y, u[j], hi[g].x);
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) t[g][j] = fma(t[g][j], u[j], lo[g].y);
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) t[g][j] = fma(t[g][j], u[j], lo[g].x);
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int j = 0; j < NP; ++j) sp[g][j] = fma(t[g][j], b[j], sp[g][j]);
+  };
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
-    a0[j] = a1[j] = a2[j] = a3[j] = 0.0;
-    // tail factor of the current l: 1 inside the grid, d^l below its first
-    // point, d^-(l+1) beyond its last
-    gstep[j] = REGION == 1 ? d[j] : (REGION == 2 ? inv[j] : 1.0);
-    gm[j] = REGION == 2 ? inv[j] : 1.0;
+    b[j] = start;
+    bp[j] = ec[j] = es[j] = oc[j] = os[j] = 0.0;
+  }
+#pragma unroll 2
+  for (int n = 0; n < nodd; ++n) {
+    if constexpr (!SIN) {
+      add(row, ec);
+      add(row + 8, oc, os);
+    } else {
+      add(row, ec, es);
+      add(row + 8, oc, os);
+    }
+    const double a = rec[n * (kMaxLmax + 1)];
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      const double t = fma(a, z[j] * b[j], -bp[j]);
+      bp[j] = b[j];
+      b[j] = t;
+    }
+    row += kEvalRow;
+  }
+  if constexpr (SIN)
+    add(row, ec, es);
+  else
+    add(row, ec);
+}
+
+template <int NP>
+__device__ __forceinline__ void interior_values(const double *cf, int L, const double *x,
+                                                const double *y, const double *z,
+                                                const double *u, double *v) {
+  double cm[NP], sm[NP], ec[NP], es[NP], oc[NP], os[NP];
+  const double *rec = c_rec_a + kMaxLmax + 1;  // A at [l = m0 + 1][m0]
+  family_sums<NP, false>(cf, L, rec, 1.0, z, u, ec, es, oc, os);
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    cm[j] = x[j];
+    sm[j] = y[j];
+    v[j] = fma(cm[j], oc[j], fma(sm[j], os[j], ec[j]));
+  }
+  auto rotate = [&]() {
+#pragma unroll
+    for (int j = 0; j < NP; ++j) {
+      const double c = cm[j] * x[j] - sm[j] * y[j];
+      sm[j] = cm[j] * y[j] + sm[j] * x[j];
+      cm[j] = c;
+    }
+  };
+#pragma unroll 1
+  for (int m0 = 2; m0 <= L; m0 += 2) {
+    cf += kEvalRow * (L + 3 - m0);  // past the L + 1 - (m0 - 2) rows of the last family
+    rec += 2 * (kMaxLmax + 1) + 2;
+    family_sums<NP, true>(cf, L - m0, rec, c_rec_start[m0], z, u, ec, es, oc, os);
+    rotate();
+#pragma unroll
+    for (int j = 0; j < NP; ++j) v[j] = fma(cm[j], ec[j], fma(sm[j], es[j], v[j]));
+    rotate();
+#pragma unroll
+    for (int j = 0; j < NP; ++j) v[j] = fma(cm[j], oc[j], fma(sm[j], os[j], v[j]));
+  }
+}
+
+// The interval's cubics src[lm][4], l <= L, into the rows of interior_values:
+// scaled, then the suffix sums of the odd columns (one thread per column,
+// cos/sin, power and parity of l).  Ends with a barrier.  (What no series
+// reads, the sine half of m = 0 and the odd column at l = L, stays unset.)
+__device__ __forceinline__ void stage_interior(double *cf, const double *src, int L) {
+  for (int lm = threadIdx.x; lm < (L + 1) * (L + 1); lm += blockDim.x) {
+    const int l = (int)sqrtf((float)lm), r = lm - l * l;  // exact: lm < 2^23
+    const int m = (r + 1) >> 1;
+    const double *c = src + 4 * lm;
+    double *d = cf + kEvalRow * (eval_family(L, m >> 1) + l - m) + 8 * (m & 1) +
+                (r > 0 && !(r & 1) ? 4 : 0);
+    const double al = g_eval_alpha[lm];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d[k] = c[k] * al;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 16 * ((L + 1) / 2); t += blockDim.x) {
+    const int f = t >> 4, m0 = 2 * f, top = L - m0 - 1;  // last row of column m0 + 1
+    double *c = cf + kEvalRow * eval_family(L, f) + 8 + (t & 7);
+    double s = 0.0;
+    for (int n = top - ((top ^ (t >> 3)) & 1); n >= 0; n -= 2) {
+      s += c[kEvalRow * n];
+      c[kEvalRow * n] = s * g_eval_beta[(m0 + n) * (kMaxLmax + 1) + m0];
+    }
+  }
+  __syncthreads();
+}
+
+// Tail pairs: the amplitudes of region 1 (below the first radial point, x d^l)
+// or 2 (beyond the last, x d^-(l+1)), column by column.
+template <int LMAX, int REGION, int NP>
+__device__ __forceinline__ void tail_values(const double *cf, int lmaxA, const double *x,
+                                            const double *y, const double *z, const double *d,
+                                            const double *inv, double *v) {
+  double gstep[NP], cm[NP], sm[NP], gm[NP];
+#pragma unroll
+  for (int j = 0; j < NP; ++j) {
+    v[j] = 0.0;
+    gstep[j] = REGION == 1 ? d[j] : inv[j];
+    gm[j] = REGION == 1 ? 1.0 : inv[j];  // tail factor at l = m
     cm[j] = 1.0;
     sm[j] = 0.0;
   }
-  // accumulate the (lm, S) term of every pair
-  auto term = [&](int lm, const double *S, const double *gl) {
-    if (REGION == 0) {
-      const double2 c01 = *reinterpret_cast<const double2 *>(cf + 4 * lm);
-      const double2 c23 = *reinterpret_cast<const double2 *>(cf + 4 * lm + 2);
-#pragma unroll
-      for (int j = 0; j < NP; ++j) {
-        a0[j] = fma(c01.x, S[j], a0[j]);
-        a1[j] = fma(c01.y, S[j], a1[j]);
-        a2[j] = fma(c23.x, S[j], a2[j]);
-        a3[j] = fma(c23.y, S[j], a3[j]);
-      }
-    } else {
-      const double c = cf[lm];
-#pragma unroll
-      for (int j = 0; j < NP; ++j) a0[j] = fma(c * gl[j], S[j], a0[j]);
-    }
-  };
-  // Normalised solid harmonics of the unit vector, m outer and l inner:
-  // q_l^m = nrm_lm Pi_l^m with Pi_m^m = (2m-1)!!, Pi_(m+1)^m = (2m+1) z Pi_m^m,
-  // Pi_l^m = ((2l-1) z Pi_(l-1)^m - (l+m-1) Pi_(l-2)^m) / (l-m) (|u| = 1);
-  // the normalisation is folded into the recursion constants (c_rec_a,
-  // c_rec_start) and the recursion runs on q~ = q / gamma (c_rec_gamma), whose
-  // scale the staged coefficients carry.  S_l0 = q_l^0; S_lm (cos, sin) =
-  // q_l^m Re/Im (x + iy)^m at lm = l^2 + 2m - 1, l^2 + 2m: the values and lm
-  // order of solid_harmonics.h, evaluated column by column so that only a few
-  // are live.
 #pragma unroll
   for (int m = 0; m <= LMAX; ++m) {
     if (m > lmaxA) break;
@@ -1126,23 +1259,14 @@ __device__ __forceinline__ void pair_values(const double *cf, int lmaxA, const d
           gl[j] *= gstep[j];
         }
       }
-      if (m == 0) {
-        term(l * l, q, gl);
-      } else {
-        double sc[NP], ss[NP];
+      const double c = cf[m == 0 ? l * l : l * l + 2 * m - 1], s = m == 0 ? 0.0 : cf[l * l + 2 * m];
 #pragma unroll
-        for (int j = 0; j < NP; ++j) {
-          sc[j] = q[j] * cm[j];
-          ss[j] = q[j] * sm[j];
-        }
-        term(l * l + 2 * m - 1, sc, gl);
-        term(l * l + 2 * m, ss, gl);
+      for (int j = 0; j < NP; ++j) {
+        v[j] = fma(c * gl[j], m == 0 ? q[j] : q[j] * cm[j], v[j]);
+        if (m > 0) v[j] = fma(s * gl[j], q[j] * sm[j], v[j]);
       }
     }
   }
-#pragma unroll
-  for (int j = 0; j < NP; ++j)
-    v[j] = REGION == 0 ? a0[j] + u[j] * (a1[j] + u[j] * (a2[j] + u[j] * a3[j])) : a0[j];
 }
 
 
@@ -1175,40 +1299,55 @@ __device__ double cubic_max_abs(const double *c) {
 // (0 <= u <= 1) inside the grid, |a_lm| first_x^l below the first radial point
 // (d^l <= first_x^l) and |a_lm| last_x^-(l+1) beyond the last.  The bucket
 // keeps l <= L, the smallest L whose dropped blocks sum to at most eval_tol.
-// Grid (max nrad + 1, natom), one warp: the lanes bound the (l, m) terms
-// lane, lane + 32, ... (every lane busy, whatever l), then lane l sums block l
-// in m order.
-__global__ void __launch_bounds__(32) bucket_lcut_kernel(PoissonDev P) {
+//
+// Then the interval's cubics, l <= L, go into the rows that interior_values
+// reads (P.rows): once per bucket and solve, not once per evaluation item.
+// Grid (max nrad + 1, natom x nbatch); the threads bound the (l, m) terms,
+// warp 0's lane l sums block l in m order.
+constexpr int kRowsThreads = 128;
+__global__ void __launch_bounds__(kRowsThreads) bucket_rows_kernel(PoissonDev P) {
   __shared__ double bound[32];
-  extern __shared__ double cterm[];  // (max_lmax + 1)^2
+  __shared__ int s_cut;
+  extern __shared__ double rows[];  // eval_rows(max_lmax) rows; first the terms
   const int bat = blockIdx.y / P.natom;  // solve of a batch
   const PoissonAtom &at = P.atoms[blockIdx.y - bat * P.natom];
-  const double *const spl = P.spl + bat * P.spl_stride;
-  const double *const amp = P.amp + bat * P.amp_stride;
-  const int b = blockIdx.x, l = threadIdx.x;
+  const int b = blockIdx.x, t = threadIdx.x;
   if (b > at.nrad) return;
   const int lmaxA = at.lmax;
   const int lsize = (lmaxA + 1) * (lmaxA + 1);
   const int region = (b == 0) ? 1 : (b == at.nrad ? 2 : 0);
-  for (int lm = l; lm < lsize; lm += 32)
-    cterm[lm] = region == 0 ? cubic_max_abs(spl + at.spl_off + ((long)(b - 1) * lsize + lm) * 4)
-                            : fabs(amp[at.amp_off + lm * 2 + (region == 1 ? 0 : 1)]);
-  __syncwarp();
-  if (l <= lmaxA) {
-    double s2 = 0.0;
-    for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) s2 = fma(cterm[lm], cterm[lm], s2);
-    const double g = region == 0 ? 1.0
-                                 : (region == 1 ? pow(at.first_x, (double)l)
-                                                : pow(at.last_x, -(double)(l + 1)));
-    bound[l] = sqrt(s2) * g;
+  const double *const cub = P.spl + bat * P.spl_stride + at.spl_off + (long)(b - 1) * lsize * 4;
+  int L = lmaxA;
+  if (P.lcut) {
+    const double *const amp = P.amp + bat * P.amp_stride + at.amp_off;
+    for (int lm = t; lm < lsize; lm += kRowsThreads)
+      rows[lm] = region == 0 ? cubic_max_abs(cub + lm * 4)
+                             : fabs(amp[lm * 2 + (region == 1 ? 0 : 1)]);
+    __syncthreads();
+    if (t <= lmaxA) {
+      double s2 = 0.0;
+      for (int lm = t * t; lm < (t + 1) * (t + 1); ++lm) s2 = fma(rows[lm], rows[lm], s2);
+      const double g = region == 0 ? 1.0
+                                   : (region == 1 ? pow(at.first_x, (double)t)
+                                                  : pow(at.last_x, -(double)(t + 1)));
+      bound[t] = sqrt(s2) * g;
+    }
+    __syncthreads();
+    if (t == 0) {
+      double dropped = 0.0;
+      while (L > 0 && dropped + bound[L] <= P.eval_tol) dropped += bound[L--];
+      P.lcut[bat * P.lcut_stride + at.bucket_off + b] = L;
+      s_cut = L;
+    }
+    __syncthreads();
+    L = s_cut;
   }
-  __syncwarp();
-  if (l == 0) {
-    double dropped = 0.0;
-    int L = lmaxA;
-    while (L > 0 && dropped + bound[L] <= P.eval_tol) dropped += bound[L--];
-    P.lcut[bat * P.lcut_stride + at.bucket_off + b] = L;
-  }
+  if (region != 0) return;
+  stage_interior(rows, cub, L);
+  double2 *out = reinterpret_cast<double2 *>(P.rows + bat * P.rows_stride + at.rows_off +
+                                             (long)(b - 1) * kEvalRow * eval_rows(lmaxA));
+  for (int e = t; e < kEvalRow / 2 * eval_rows(L); e += kRowsThreads)
+    out[e] = reinterpret_cast<const double2 *>(rows)[e];
 }
 
 // TAILS = false: the interior items [0, nitems_inner) (region 0 only, so the
@@ -1217,9 +1356,9 @@ __global__ void __launch_bounds__(32) bucket_lcut_kernel(PoissonDev P) {
 // instance carries no batch offsets (its registers, and occupancy, stay those
 // the recursion was tuned at)
 template <int LMAX, bool TAILS, bool BATCH>
-// Four 256-thread CTAs per SM (64 registers, 20 bytes spilled): 32 resident
-// warps instead of 24 at the compiler's 76 registers; the FP64 pipe, busy 77 %
-// at 24 warps, throttles less often (C20H42 evaluation 3 % faster).
+// Four 128-thread CTAs per SM (128 registers): 16 warps with eight independent
+// products each.  Measured at C12H26: two pairs per thread at 64 registers
+// 3.74 ms, three at 80 3.77 ms, four at 96 3.87 ms and at 128 3.55 ms.
 __global__ void __launch_bounds__(kEvalChunkMax / kEvalPerThread, 4)
 eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
                   const double *__restrict__ gy, const double *__restrict__ gz) {
@@ -1232,29 +1371,29 @@ eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
   const long bat = BATCH ? (long)blockIdx.y : 0;  // solve of a batch
   // l-blocks kept for this bucket (all unless a truncation tolerance is set)
   const int lcut = P.lcut ? P.lcut[bat * P.lcut_stride + at.bucket_off + it.bucket] : lmaxA;
-  const int lkeep = (lcut + 1) * (lcut + 1);
-  // staged with the recursion's scale gamma_lm (see c_rec_gamma)
-  if (region == 0) {
-    const double *src =
-        P.spl + bat * P.spl_stride + at.spl_off + (long)(it.bucket - 1) * lsize * 4;
-    for (int e = threadIdx.x; e < lkeep * 4; e += blockDim.x) cf[e] = src[e] * g_rec_gamma[e >> 2];
-  } else {
+  if (region == 0) {  // 16-byte copies in flight while the pairs are read
+    const double *src = P.rows + bat * P.rows_stride + at.rows_off +
+                        (long)(it.bucket - 1) * kEvalRow * eval_rows(lmaxA);
+    for (int e = threadIdx.x; e < kEvalRow / 2 * eval_rows(lcut); e += blockDim.x)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(cf + 2 * e)),
+                   "l"(src + 2 * e)
+                   : "memory");
+  } else {  // with the recursion's scale gamma_lm (see g_rec_gamma)
     const double *src = P.amp + bat * P.amp_stride + at.amp_off;
-    for (int e = threadIdx.x; e < lkeep; e += blockDim.x)
+    for (int e = threadIdx.x; e < (lcut + 1) * (lcut + 1); e += blockDim.x)
       cf[e] = src[2 * e + (region == 1 ? 0 : 1)] * g_rec_gamma[e];
   }
-  __syncthreads();
-  // thread t evaluates the pairs t and t + blockDim.x of the item (the
-  // second may be absent: it then repeats the first and is not stored)
+  // thread t evaluates the pairs t + j blockDim.x of the item (an absent one
+  // repeats the item's first and is not stored)
   const int t = threadIdx.x;
-  if (t >= it.count) return;
   int pidx[kEvalPerThread];
   double x[kEvalPerThread], y[kEvalPerThread], z[kEvalPerThread], d[kEvalPerThread],
       inv[kEvalPerThread], u[kEvalPerThread], v[kEvalPerThread];
 #pragma unroll
   for (int j = 0; j < kEvalPerThread; ++j) {
     const int e = t + j * (int)blockDim.x;
-    const long slot = at.pair_off + it.start + (e < it.count ? e : t);
+    const long slot = at.pair_off + it.start + (e < it.count ? e : 0);
     pidx[j] = P.pairs[slot];
     const int p = pidx[j];
     const double dx = gx[p] - at.cx, dy = gy[p] - at.cy, dz = gz[p] - at.cz;
@@ -1272,12 +1411,15 @@ eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
     y[j] = dy * inv[j];
     z[j] = dz * inv[j];
   }
+  if (!TAILS) asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();
+  if (t >= it.count) return;
   if (!TAILS)
-    pair_values<LMAX, 0, kEvalPerThread>(cf, lcut, x, y, z, d, inv, u, v);
+    interior_values<kEvalPerThread>(cf, lcut, x, y, z, u, v);
   else if (region == 1)
-    pair_values<LMAX, 1, kEvalPerThread>(cf, lcut, x, y, z, d, inv, u, v);
+    tail_values<LMAX, 1, kEvalPerThread>(cf, lcut, x, y, z, d, inv, v);
   else
-    pair_values<LMAX, 2, kEvalPerThread>(cf, lcut, x, y, z, d, inv, u, v);
+    tail_values<LMAX, 2, kEvalPerThread>(cf, lcut, x, y, z, d, inv, v);
 #pragma unroll
   for (int j = 0; j < kEvalPerThread; ++j) {
     const int e = t + j * (int)blockDim.x;
@@ -1321,13 +1463,12 @@ cudaError_t launch_eval_l(const PoissonDev &P, int npoint, const double *x,
                           const double *y, const double *z, double *out, int acc,
                           cudaStream_t s) {
   if (P.items && P.nitems > 0) {
-    if (P.lcut) {
-      bucket_lcut_kernel<<<dim3(P.max_nrad + 1, P.natom * P.nbatch), 32,
-                           (size_t)(P.max_lmax + 1) * (P.max_lmax + 1) * sizeof(double), s>>>(P);
-      cudaError_t e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
-    }
-    const size_t smem = (size_t)(L + 1) * (L + 1) * 4 * sizeof(double);
+    bucket_rows_kernel<<<dim3(P.max_nrad + 1, P.natom * P.nbatch), kRowsThreads,
+                         (size_t)kEvalRow * eval_rows(P.max_lmax) * sizeof(double), s>>>(P);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const size_t smem = (size_t)kEvalRow * eval_rows(L) * sizeof(double);
+    const size_t smem_tail = (size_t)(L + 1) * (L + 1) * sizeof(double);
     const dim3 gin(P.nitems_inner, P.nbatch), gtail(P.nitems - P.nitems_inner, P.nbatch);
     const int kT = P.eval_chunk / kEvalPerThread;
     if (P.nitems_inner > 0) {
@@ -1338,11 +1479,11 @@ cudaError_t launch_eval_l(const PoissonDev &P, int npoint, const double *x,
     }
     if (P.nitems > P.nitems_inner) {
       if (P.nbatch > 1)
-        eval_pairs_kernel<L, true, true><<<gtail, kT, smem, s>>>(P, x, y, z);
+        eval_pairs_kernel<L, true, true><<<gtail, kT, smem_tail, s>>>(P, x, y, z);
       else
-        eval_pairs_kernel<L, true, false><<<gtail, kT, smem, s>>>(P, x, y, z);
+        eval_pairs_kernel<L, true, false><<<gtail, kT, smem_tail, s>>>(P, x, y, z);
     }
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     pairs_reduce_kernel<<<dim3((npoint + 255) / 256, P.nbatch), 256, 0, s>>>(P, npoint, out,
                                                                              acc);
@@ -1354,6 +1495,8 @@ cudaError_t launch_eval_l(const PoissonDev &P, int npoint, const double *x,
 }
 
 }  // namespace
+
+size_t eval_rows_doubles(int lmax) { return (size_t)kEvalRow * eval_rows(lmax); }
 
 // Uploads the constant tables to the current device.  Called by every Poisson
 // plan construction (which allocates and copies far more): uploading per plan
@@ -1394,20 +1537,25 @@ cudaError_t poisson_init_constants() {
     }
     // rescaled recursion: gamma per (l, m), A = a gamma_(l-1) / gamma_l, and
     // gamma laid out per lm (cos and sin columns share it)
-    std::vector<double> gam(K * K, 1.0), A(K * K, 0.0), gam_lm(K * K, 1.0);
+    std::vector<double> gam(K * K, 1.0), A(K * K, 0.0), gam_lm(K * K, 1.0), alpha(K * K, 1.0),
+        beta(K * K, 1.0);
     for (int m = 0; m <= kMaxLmax; ++m)
       for (int l = m; l <= kMaxLmax; ++l) {
         if (l >= m + 2) gam[l * K + m] = rb[l * K + m] * gam[(l - 2) * K + m];
         if (l > m) A[l * K + m] = ra[l * K + m] * gam[(l - 1) * K + m] / gam[l * K + m];
+        beta[l * K + m] = (2 * l + 1) * gam[l * K + m] / nr(l, m);
+        const double al = m % 2 == 0 ? gam[l * K + m] : nr(l, m);
         if (m == 0) {
           gam_lm[l * l] = gam[l * K];
+          alpha[l * l] = al;
         } else {
-          gam_lm[l * l + 2 * m - 1] = gam[l * K + m];
-          gam_lm[l * l + 2 * m] = gam[l * K + m];
+          gam_lm[l * l + 2 * m - 1] = gam_lm[l * l + 2 * m] = gam[l * K + m];
+          alpha[l * l + 2 * m - 1] = alpha[l * l + 2 * m] = al;
         }
       }
+    if ((e = cudaMemcpyToSymbol(g_eval_alpha, alpha.data(), alpha.size() * sizeof(double))) != cudaSuccess) return e;
+    if ((e = cudaMemcpyToSymbol(g_eval_beta, beta.data(), beta.size() * sizeof(double))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_rec_a, A.data(), A.size() * sizeof(double))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(c_rec_gamma, gam_lm.data(), gam_lm.size() * sizeof(double))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(c_rec_start, st.data(), st.size() * sizeof(double))) != cudaSuccess) return e;
     if ((e = cudaMemcpyToSymbol(g_rec_gamma, gam_lm.data(), gam_lm.size() * sizeof(double))) !=
         cudaSuccess)

@@ -27,6 +27,7 @@ struct PoissonAtom {
   int bucket_off;  // [nrad + 1] buckets: 0 left tail, 1 + j interval j, nrad right tail
   int sys_off;     // radial system of (this atom, l) = sys_off + l
   long pair_off;   // this atom's slice of the (atom, point) pair arrays
+  long rows_off;   // evaluation rows: [nrad - 1][eval_rows_doubles(lmax)]
   long scr_off;    // radial-solve scratch: [3 nrad][lsize]
 };
 
@@ -37,7 +38,7 @@ struct EvalItem {
 };
 constexpr int kEvalChunk = 128;     // default pairs per item
 constexpr int kEvalChunkMax = 512;  // largest item (PoissonDev::eval_chunk)
-constexpr int kEvalPerThread = 2;   // pairs evaluated by one thread
+constexpr int kEvalPerThread = 4;   // pairs evaluated by one thread
 
 // Radial table slots (each nrad long, at rad_off + slot * nrad).
 enum : int {
@@ -68,6 +69,7 @@ struct PoissonDev {
   double *ytab = nullptr;
   double *proj = nullptr;
   double *spl = nullptr;
+  double *rows = nullptr;  // spl as the interior evaluation reads it
   double *amp = nullptr;
   double *raw_y = nullptr;
   double *raw_dt = nullptr;
@@ -91,7 +93,7 @@ struct PoissonDev {
   long npair = 0;
   int nitems = 0;
   int nitems_inner = 0;        // items [0, nitems_inner) lie inside their atom's grid
-  int eval_chunk = kEvalChunk;  // pairs per item (<= kEvalChunkMax); CTA = chunk / 2 threads
+  int eval_chunk = kEvalChunk;  // pairs per item (<= kEvalChunkMax); CTA = chunk / 4 threads
   int *pairs = nullptr;        // point index, bucket-sorted per atom
   double2 *pair_u = nullptr;   // (u, 1/d) of each interior pair (slot order)
   EvalItem *items = nullptr;
@@ -110,7 +112,7 @@ struct PoissonDev {
   // doubles (ints for lcut) apart.  nbatch = 1: one solve, strides unused.
   int nbatch = 1;
   long batch_ld = 0;
-  long proj_stride = 0, spl_stride = 0, amp_stride = 0, lcut_stride = 0, pairv_stride = 0;
+  long proj_stride = 0, spl_stride = 0, rows_stride = 0, amp_stride = 0, lcut_stride = 0, pairv_stride = 0;
 };
 
 // Radial stage of the pipeline.  The default is the Poisson equation
@@ -125,6 +127,9 @@ struct RadialOp {
   double e = 0.0, de = 0.0;      // orbital energy and its correction
   bool zero_bc = false;          // u = 0 at the first and last radial point
 };
+
+// Doubles per spline interval of the evaluation rows.
+size_t eval_rows_doubles(int lmax);
 
 // Uploads the Hermite FEM integral tables and solid-harmonic norms to
 // constant memory (idempotent, per device).
