@@ -38,6 +38,8 @@ struct DevBuf {
     if (e == cudaSuccess) n = count;
     return e;
   }
+  // at least `count` elements; a buffer that is large enough is kept
+  cudaError_t reserve(size_t count) { return n >= count ? cudaSuccess : alloc(count); }
   cudaError_t upload(const T *h, size_t count, cudaStream_t s) {
     cudaError_t e = alloc(count);
     if (e != cudaSuccess || count == 0) return e;

@@ -56,3 +56,30 @@ def test_truncated_potential(oracle, basis_library, elements, lmax):
         v = fb.coulomb_potential(rho)
         # each of the three atoms drops at most tol; rounding as above
         assert float((v - full).abs().max()) <= 3 * tol + 1e-12 * float(full.abs().max()), tol
+
+
+@pytest.mark.parametrize('precision', ['fp64', 'int8x4'])
+@pytest.mark.parametrize('nrad,nang', [(5, 6), (40, 110)])
+def test_moved_plan_equals_a_new_one(oracle, basis_library, elements, precision, nrad, nang):
+    import torch
+    import napmo_b200 as nb
+    lmax = nb.lebedev_get_order(nang) // 2
+    basis, grid, og = _grids(oracle, basis_library, elements, nrad, nang)
+    fb = nb.FockBuilder(grid, basis, lmax, precision=precision)
+    rho = torch.as_tensor(np.stack([_density(og, k) for k in range(2)])).cuda()
+    fb.coulomb_potentials(rho)
+    R = np.array([xyz for _, xyz in H2O]) / 0.52917724924
+    of = [int(np.argmin(((R - o) ** 2).sum(1))) for o in basis.origins()]
+    # far apart (tail pairs grow), close together (they vanish), back
+    for scale in (6.0, 0.8, 1.0):
+        grid.set_centers(R * scale)
+        basis.set_origins((R * scale)[of])
+        fb.refresh()
+        moved = fb.coulomb_potentials(rho)
+        atoms = [(s, tuple(np.array(x) * scale)) for s, x in H2O]
+        ms, fresh = product_system(atoms, nrad=nrad, nang=nang)
+        fresh.set_centers(R * scale)  # the very same centres, to the last bit
+        ms['e-']['basis'].set_origins((R * scale)[of])
+        new = nb.FockBuilder(fresh, ms['e-']['basis'], lmax, precision=precision)
+        assert torch.equal(moved, new.coulomb_potentials(rho)), scale
+        assert torch.equal(fb.coulomb_potential(rho[0]), moved[0])
