@@ -44,6 +44,9 @@ struct PoissonPlan {
   DevBuf<int> mol_atom_off, mol_point_off, sys_atom, sys_l;
   DevBuf<double> rad, ytab, proj, spl, rows, amp, raw_y, raw_dt, lu, lmul;
   DevBuf<int> lpiv;
+  DevBuf<double> gop;  // radial operators (see PoissonDev)
+  DevBuf<RadialGroup> groups;
+  DevBuf<int> group_atom;
   DevBuf<double> rscr;  // radial-solve scratch of one solve
   DevBuf<double> pg;    // projection scratch of one solve (rho wb w per point)
   DevBuf<int> pairs;
@@ -90,6 +93,91 @@ static void ytable(const std::vector<double> &ang, int nang, int lmax,
       for (int k = 1; k < lsize; ++k) y[k] = work[k - 1];
     }
   }
+}
+
+// The radial operators of a plan whose atoms (h_atoms, d.atoms) and radial tables
+// are set: one set per distinct radial grid, whatever its atoms.  *use = false,
+// with nothing built, for grids beyond kRadialOpMax points or operators beyond
+// kRadialOpBytes in all: those plans substitute per solve.
+constexpr size_t kRadialOpBytes = 512ull << 20;
+static int build_radial_operators(PoissonPlan *plan, const std::vector<double> &rad,
+                                  cudaStream_t s, bool *use) {
+  PoissonDev &d = plan->d;
+  std::vector<PoissonAtom> &ha = plan->h_atoms;
+  *use = false;
+  if (d.natom == 0 || d.max_nrad > kRadialOpMax) return kOk;
+  // atoms by radial grid (radius, weight and the three derivatives: the first
+  // five tables), then by lmax
+  auto less = [&](int a, int b) {
+    if (ha[a].nrad != ha[b].nrad) return ha[a].nrad < ha[b].nrad;
+    const int c = std::memcmp(&rad[ha[a].rad_off], &rad[ha[b].rad_off],
+                              5 * (size_t)ha[a].nrad * sizeof(double));
+    return c != 0 ? c < 0 : false;
+  };
+  std::map<int, std::map<int, std::vector<int>>, decltype(less)> kinds(less);
+  for (int a = 0; a < d.natom; ++a) kinds[a][ha[a].lmax].push_back(a);
+  std::vector<RadialGroup> groups;
+  std::vector<int> order, sys_atom, sys_l;
+  size_t total = 0;
+  d.max_group_cols = 0;
+  for (auto &kind : kinds) {
+    const int n = ha[kind.first].nrad;
+    int top = 0;  // an atom with the kind's largest lmax
+    for (auto &by : kind.second) {
+      const int lmax = by.first, count = (int)by.second.size();
+      for (int l = 0; l <= lmax; ++l)
+        groups.push_back(RadialGroup{(int)order.size(), count, l});
+      for (int a : by.second) {
+        order.push_back(a);
+        ha[a].gop_off = (long)total;
+      }
+      top = by.second[0];
+      d.max_group_cols = std::max(d.max_group_cols, count * (2 * lmax + 1));
+    }
+    for (int l = 0; l <= ha[top].lmax; ++l) {
+      sys_atom.push_back(top);
+      sys_l.push_back(l);
+    }
+    total += (size_t)(ha[top].lmax + 1) * radial_op_rows(n) * radial_op_ld(n);
+  }
+  if (total * sizeof(double) > kRadialOpBytes || groups.size() > 65535) return kOk;
+  // one temporary: the kinds' systems, their LU factors and the table's scratch
+  const int nk = (int)sys_atom.size();
+  const size_t rows = (size_t)nk * d.lu_stride;
+  const size_t doubles = rows * (kW + kKL) + radial_op_tmp_doubles(nk, d.max_nrad);
+  DevBuf<double> tmp;
+  DevBuf<int> itmp;
+  std::vector<int> sys(sys_atom);
+  sys.insert(sys.end(), sys_l.begin(), sys_l.end());
+  NAPMO_TRY_CUDA(tmp.alloc(doubles), "alloc radial operators");
+  NAPMO_TRY_CUDA(itmp.alloc(2 * (size_t)nk + rows), "alloc radial operators");
+  NAPMO_TRY_CUDA(cudaMemcpyAsync(itmp.p, sys.data(), sys.size() * sizeof(int),
+                                 cudaMemcpyHostToDevice, s),
+                 "upload");
+  NAPMO_TRY_CUDA(plan->gop.alloc(total), "alloc radial operators");
+  NAPMO_TRY_CUDA(cudaMemsetAsync(plan->gop.p, 0, total * sizeof(double), s), "radial operators");
+  NAPMO_TRY_CUDA(plan->groups.upload(groups, s), "upload");
+  NAPMO_TRY_CUDA(plan->group_atom.upload(order, s), "upload");
+  NAPMO_TRY_CUDA(cudaMemcpyAsync(plan->atoms.p, ha.data(), ha.size() * sizeof(PoissonAtom),
+                                 cudaMemcpyHostToDevice, s),
+                 "upload atoms");
+  PoissonDev k = d;
+  k.gop = plan->gop.p;
+  k.nsys = nk;
+  k.sys_atom = itmp.p;
+  k.sys_l = itmp.p + nk;
+  k.lpiv = itmp.p + 2 * nk;
+  k.lu = tmp.p;
+  k.lmul = k.lu + rows * kW;
+  NAPMO_TRY_CUDA(launch_poisson_factor(k, s), "radial LU");
+  NAPMO_TRY_CUDA(launch_radial_operators(k, k.lmul + rows * kKL, s), "radial operators");
+  NAPMO_TRY_CUDA(cudaStreamSynchronize(s), "radial operators");
+  d.gop = plan->gop.p;
+  d.groups = plan->groups.p;
+  d.group_atom = plan->group_atom.p;
+  d.ngroup = (int)groups.size();
+  *use = true;
+  return kOk;
 }
 
 int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
@@ -222,8 +310,11 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
   d.rscr = plan->rscr.p;
   d.pg = plan->pg.p;
   d.npair = pairs;
-  // LU factors of the radial systems (they depend on the grid only)
   d.lu_stride = 2 * d.max_nrad;
+  bool use = false;
+  int st = build_radial_operators(plan, rad, s, &use);
+  if (st != kOk || use) return st;
+  // LU factors of the radial systems (they depend on the grid only)
   NAPMO_TRY_CUDA(plan->lu.alloc((size_t)d.nsys * d.lu_stride * kW), "alloc radial LU");
   NAPMO_TRY_CUDA(plan->lmul.alloc((size_t)d.nsys * d.lu_stride * kKL), "alloc radial LU");
   NAPMO_TRY_CUDA(plan->lpiv.alloc((size_t)d.nsys * d.lu_stride), "alloc radial LU");
@@ -583,7 +674,9 @@ int run_poisson_many(BeckeGrid *g, PoissonPlan *p, int k, const double *rho_dev,
   int st = select_pair_lists(p, g, keep, key, s);
   if (st) return st;
   const PoissonDev &d = p->d;
-  const size_t nd = p->proj.n + p->spl.n + p->rows.n + p->amp.n + p->pair_v.n + p->rscr.n + p->pg.n;
+  const size_t nscr = d.gop ? 0 : p->rscr.n;  // the operators need no scratch
+  const size_t nd = p->proj.n + p->spl.n + p->rows.n + p->amp.n + p->pair_v.n + nscr +
+                    p->pg.n;
   const size_t per = nd * sizeof(double) + p->lcut.n * sizeof(int);
   // grid limits: the projection and truncation launches use natom x B blocks
   // in y/z, the radial one B in y
@@ -609,12 +702,12 @@ int run_poisson_many(BeckeGrid *g, PoissonPlan *p, int k, const double *rho_dev,
   P.amp_stride = (long)p->amp.n;
   P.pairv_stride = (long)p->pair_v.n;
   P.lcut_stride = (long)p->lcut.n;
-  P.rscr_stride = (long)p->rscr.n;
+  P.rscr_stride = (long)nscr;
   double *ws = (double *)p->batch_ws.p;
-  P.rows = ws;  // first: its 16-byte copies need the allocation's alignment
-  P.proj = P.rows + P.rows_stride * B;
-  P.spl = P.proj + P.proj_stride * B;
-  P.amp = P.spl + P.spl_stride * B;
+  P.rows = ws;  // rows and spl first: 16-byte accesses
+  P.spl = P.rows + P.rows_stride * B;
+  P.proj = P.spl + P.spl_stride * B;
+  P.amp = P.proj + P.proj_stride * B;
   P.pair_v = P.amp + P.amp_stride * B;
   P.rscr = P.pair_v + P.pairv_stride * B;
   P.pg_stride = (long)p->pg.n;

@@ -6,12 +6,16 @@
 //    AtomicGrid::spherical_expansion, src/grid/atomic_grid.cpp:82-136).
 // 2. radial:   the Hermite FEM matrix of u'' + b u' + a u = f on the uniform
 //    t-axis depends on (atom, l) only: it is assembled and factored by banded
-//    LU with partial pivoting once per grid (radial_factor_kernel).  Per solve,
-//    one thread per (l, m) column builds the cubic spline of f_lm, the
-//    transformed FEM right-hand side and Dirichlet values, and substitutes
-//    (radial_kernel; reference: poisson_solver.py:42-118, ode2.py,
-//    src/horton/ode2.cpp:232-321; the reference solves each (l, m) with
-//    scipy's sparse LU).  The solution splines are written as scaled cubic
+//    LU with partial pivoting once per grid (radial_factor_kernel).  The cubic
+//    spline of f_lm, the transformed FEM right-hand side, the Dirichlet values
+//    and the substitution are linear in f_lm (reference: poisson_solver.py:
+//    42-118, ode2.py, src/horton/ode2.cpp:232-321; the reference solves each
+//    (l, m) with scipy's sparse LU), so their composition is tabulated once per
+//    radial grid and l by solving for unit f (radial_kernel<true>), and a solve
+//    is one FP64 tensor product per (radial grid, l) (radial_apply_kernel).
+//    Radial grids beyond kRadialOpMax points and the Becke-Dickson correction,
+//    whose matrix changes with every call, substitute per solve
+//    (radial_kernel<false>).  The solution splines are written as scaled cubic
 //    coefficients for step 3 and as raw (y, dy/dt) for the Python API.
 // 3. evaluate: v(p) = sum_A sum_lm s_lm(|p - A|) sqrt(2l+1)/sqrt(4 pi)
 //    S_lm(p - A) / |p - A|^l for every point and every atom (the potential
@@ -426,7 +430,8 @@ __global__ void radial_factor_kernel(PoissonDev P, RadialOp op) {
   for (int e = tid; e < n2 * kW; e += nt) lu[e] = band[e];
 }
 
-// Radial solve.  CTA = (system (atom, l), group of solves of the batch);
+// Radial solve by substitution.  CTA = (system (atom, l), group of solves of the
+// batch);
 // thread = one column (solve, m), lm = l^2 + m.  A column is a chain of
 // dependent steps: the Thomas sweep of the spline through f_lm (with the
 // boundary moments), the forward elimination of the FEM right-hand side with
@@ -448,6 +453,10 @@ __global__ void radial_factor_kernel(PoissonDev P, RadialOp op) {
 // q + 1 (q = row / 2; 0 where a node does not exist).  The arithmetic is that
 // of poisson_solver.py:42-118 and ode2.py (spline, FEM assembly, banded LU
 // solve with partial pivoting), up to rounding.
+// TABLE: the columns are the unit vectors f = e_j of the system's radial grid,
+// read from an identity matrix (ldi x ldi), and column j of the radial operator
+// leaves instead of the spline tables (over the eliminated rows, which the back
+// substitution has read by then).
 constexpr int kRadialThreads = 128;
 constexpr int kRing = 32;  // doubles per thread: one ring of 32 or two of 16
 
@@ -475,15 +484,19 @@ __device__ __forceinline__ void ring_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-__global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, RadialOp op) {
+template <bool TABLE>
+__global__ void __launch_bounds__(kRadialThreads)
+radial_kernel(PoissonDev P, RadialOp op, const double *__restrict__ ident, int ldi, double *tab) {
   extern __shared__ double sm[];
   const int sys = blockIdx.x;
   const PoissonAtom at = P.atoms[P.sys_atom[sys]];
   const int l = P.sys_l[sys];
-  const int ncol = 2 * l + 1, spc = radial_solves_per_cta(l, blockDim.x);
-  const int bat0 = blockIdx.y * spc;
-  if (bat0 >= P.nbatch) return;  // the whole CTA
   const int n = at.nrad, n2 = 2 * n;
+  const int ncol = TABLE ? 1 : 2 * l + 1;
+  const int spc = TABLE ? blockDim.x : radial_solves_per_cta(l, blockDim.x);
+  const int nbatch = TABLE ? n : P.nbatch;
+  const int bat0 = blockIdx.y * spc;
+  if (bat0 >= nbatch) return;  // the whole CTA
   const int lsize = (at.lmax + 1) * (at.lmax + 1);
   const long xmax = n - 1;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -531,12 +544,16 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
   __syncthreads();
   const int sidx = tid / ncol, m = tid - sidx * ncol;
   const long bat = bat0 + sidx;
-  if (sidx >= spc || bat >= P.nbatch) return;  // no barrier below
+  if (sidx >= spc || bat >= nbatch) return;  // no barrier below
   const int lm = l * l + m;
-  const int ls = lsize;
-  const double *Y = P.proj + bat * P.proj_stride + at.proj_off + lm;  // f_lm(r_i) at Y[i ls]
-  double *S = P.rscr + bat * P.rscr_stride + at.scr_off + lm;        // slot s at S[s ls]
-  double *E = S + n * ls;                                             // eliminated rows
+  // f_lm(r_i) at Y[i ly], scratch slot s (t-derivatives) at S[s ls], eliminated
+  // row s at E[s le]
+  const int ly = TABLE ? ldi : lsize, ls = TABLE ? ldi : lsize;
+  const int le = TABLE ? radial_op_ld(n) : lsize;
+  const double *Y = TABLE ? ident + bat : P.proj + bat * P.proj_stride + at.proj_off + lm;
+  double *S = TABLE ? tab + (long)sys * ldi * ldi + bat
+                    : P.rscr + bat * P.rscr_stride + at.scr_off + lm;
+  double *E = TABLE ? P.gop + at.gop_off + (long)l * radial_op_rows(n) * le + bat : S + n * ls;
   double *q = ring + tid;  // this thread's ring: slot s at q[s nt]
   constexpr int R1 = kRing, R2 = kRing / 2;  // ring lengths; lookahead R - 2
   auto back2 = [](int slot, int R) { return slot >= 2 ? slot - 2 : slot + R - 2; };
@@ -549,10 +566,10 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
   double smax = 0.0, smin = 0.0, prev;
   {
     for (int s = 1; s < R1 - 1; ++s) {
-      ring_copy(q + s * nt, Y + (s + 1 < n ? s + 1 : 0) * ls, s + 1 < n);
+      ring_copy(q + s * nt, Y + (s + 1 < n ? s + 1 : 0) * ly, s + 1 < n);
       ring_commit();
     }
-    double ym = Y[0], yc = Y[ls];
+    double ym = Y[0], yc = Y[ly];
     prev = (3.0 * (yc - ym)) * rden[0];
     S[0] = prev;
     if (moments) {
@@ -562,7 +579,7 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     int slot = 1;
     for (int i = 1; i < n; ++i) {
       const int j = i + R1 - 1;  // y index the refill brings, for step i + R1 - 2
-      ring_copy(q + back2(slot, R1) * nt, Y + (j < n ? j : 0) * ls, j < n);
+      ring_copy(q + back2(slot, R1) * nt, Y + (j < n ? j : 0) * ly, j < n);
       ring_commit();
       ring_wait<R1 - 2>();
       const double yn = q[slot * nt];
@@ -639,13 +656,13 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     return fma(co, o[5], acc);
   };
   node_f(0, Y[0], S[0], be, bo);
-  node_f(1, Y[ls], S[ls], ce, co);
+  node_f(1, Y[ly], S[ls], ce, co);
   double w0 = rhs_row(0), w1 = rhs_row(1), w2, w3;  // rows k .. k + 3
   ae = be;
   ao = bo;
   be = ce;
   bo = co;
-  node_f(2, n > 2 ? Y[2 * ls] : 0.0, n > 2 ? S[2 * ls] : 0.0, ce, co);
+  node_f(2, n > 2 ? Y[2 * ly] : 0.0, n > 2 ? S[2 * ls] : 0.0, ce, co);
   w2 = rhs_row(2);
   w3 = rhs_row(3);
   auto step = [&](int k) {
@@ -660,7 +677,7 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     w1 = fma(-m0, rk, w1);
     w2 = fma(-m1, rk, w2);
     w3 = fma(-m2, rk, w3);
-    E[k * ls] = rk;
+    E[(long)k * le] = rk;
     w0 = w1;
     w1 = w2;
     w2 = w3;
@@ -670,7 +687,7 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     // the two rings
     for (int s = 0; s < R2 - 2; ++s) {
       const int i = s + 3;
-      ring_copy(qa + s * nt, Y + (i < n ? i : 0) * ls, i < n);
+      ring_copy(qa + s * nt, Y + (i < n ? i : 0) * ly, i < n);
       ring_copy(qb + s * nt, S + (i < n ? i : 0) * ls, i < n);
       ring_commit();
     }
@@ -678,7 +695,7 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     for (int it = 0; it < n; ++it) {
       const int k = 2 * it, i = it + 3 + (R2 - 2);  // node of the refill
       const int rs = back2(slot, R2);
-      ring_copy(qa + rs * nt, Y + (i < n ? i : 0) * ls, i < n);
+      ring_copy(qa + rs * nt, Y + (i < n ? i : 0) * ly, i < n);
       ring_copy(qb + rs * nt, S + (i < n ? i : 0) * ls, i < n);
       ring_commit();
       step(k);
@@ -709,13 +726,13 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
   double dnext = 0.0;  // dy/dt of node j + 1
   for (int t = 0; t < R1 - 2; ++t) {
     const int i = n2 - 1 - t;
-    ring_copy(q + t * nt, E + (i >= 0 ? i : 0) * ls, i >= 0);
+    ring_copy(q + t * nt, E + (long)(i >= 0 ? i : 0) * le, i >= 0);
     ring_commit();
   }
   int slot = 0;
   for (int i = n2 - 1; i >= 0; --i) {
     const int j = i - (R1 - 2);
-    ring_copy(q + back2(slot, R1) * nt, E + (j >= 0 ? j : 0) * ls, j >= 0);
+    ring_copy(q + back2(slot, R1) * nt, E + (long)(j >= 0 ? j : 0) * le, j >= 0);
     ring_commit();
     ring_wait<R1 - 2>();
     const double ei = q[slot * nt];
@@ -731,12 +748,16 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     if ((i & 1) == 0) {
       const int jn = i / 2;
       const double d0 = (x1 * rj1[jn]) * j1[jn];
-      if (P.raw_y) {
+      if (TABLE) {
+        E[(long)i * le] = x;
+        E[(long)(i + 1) * le] = d0;
+      } else if (P.raw_y) {
         const long o = at.raw_off + (long)lm * n + jn;
         P.raw_y[o] = x;
         P.raw_dt[o] = d0;
       }
-      if (jn < n - 1) {
+      if (TABLE) {
+      } else if (jn < n - 1) {
         const double z = x2 - x;
         double *cf = spl + (long)jn * lsize * 4;
         cf[0] = x * fl;
@@ -746,7 +767,7 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
       } else {
         amp[1] = x * pow(at.last_x, (double)(l + 1)) * fl;
       }
-      if (i == 0) amp[0] = x / pow(at.first_x, (double)l) * fl;
+      if (!TABLE && i == 0) amp[0] = x / pow(at.first_x, (double)l) * fl;
       dnext = d0;
     }
     x6 = x5;
@@ -757,6 +778,130 @@ __global__ void __launch_bounds__(kRadialThreads) radial_kernel(PoissonDev P, Ra
     x1 = x;
   }
   ring_wait<0>();
+}
+
+__global__ void identity_kernel(double *a, int ld) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  if (j < ld) a[(long)i * ld + j] = i == j;
+}
+
+// Radial solve by operator: X = G_l F for the columns (solve, atom, m) of one
+// group (atoms of one radial grid and lmax), G_l [2 nrad][nrad].  CTA = (group,
+// 32 columns): F is staged in shared memory, a warp forms 32 rows at a time FP64 tensor pipe with G's fragments read straight from L2 (each is used once per
+// CTA), and X, staged in shared memory, leaves as the cubic of
+// every interval and the tail amplitudes.  Every column's sums run over the
+// radial points in order, whatever the batch.
+// Substituting instead costs 6 nrad dependent steps of some 180 ns with one
+// warp per (atom, l); this costs 4 nrad^2 operations per column, all
+// independent.  B200, substitution -> product: H2O 50 x 110 52 -> 13 us, C5H12
+// 75 x 194 81 -> 24, C12H26 100 x 302 111 -> 36, C20H42 215 -> 62, HCN 100 x 302
+// x 35 solves 151 -> 75.  kRadialOpMax: beyond it F and X outgrow the shared
+// memory.
+constexpr int kApplyCols = 32, kApplyThreads = 256;
+constexpr int kApplyLdf = kApplyCols + 4, kApplyLdx = kApplyCols + 1;
+
+__host__ __device__ constexpr size_t radial_apply_doubles(int n) {
+  return (size_t)radial_op_ld(n) * kApplyLdf + (size_t)radial_op_rows(n) * kApplyLdx;
+}
+
+__global__ void __launch_bounds__(kApplyThreads, 2) radial_apply_kernel(PoissonDev P) {
+  extern __shared__ double sm[];
+  const RadialGroup gr = P.groups[blockIdx.y];
+  const int l = gr.l, ncol = 2 * l + 1;
+  const int ncols = ncol * gr.natom * P.nbatch;  // natom x nbatch < 2^16, ncol <= 41
+  const int c0 = blockIdx.x * kApplyCols;
+  if (c0 >= ncols) return;
+  constexpr int W = kApplyThreads / 32;
+  const PoissonAtom &rep = P.atoms[P.group_atom[gr.first]];
+  const int n = rep.nrad, ld = radial_op_ld(n), rows = radial_op_rows(n);
+  const int lsize = (rep.lmax + 1) * (rep.lmax + 1);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  double *fs = sm;                   // [ld][kApplyLdf]
+  double *xs = fs + ld * kApplyLdf;  // [rows][kApplyLdx]
+  // this lane's column: solve bat, atom at, lm
+  const bool live = c0 + lane < ncols;
+  const int c = live ? c0 + lane : 0;
+  const int ba = c / ncol, lm = l * l + c - ba * ncol;
+  const long bat = ba / gr.natom;
+  const PoissonAtom &at = P.atoms[P.group_atom[gr.first + ba - (int)bat * gr.natom]];
+  const double *Y = P.proj + bat * P.proj_stride + at.proj_off + lm;
+#pragma unroll 8
+  for (int i = wid; i < ld; i += W)
+    fs[i * kApplyLdf + lane] = live && i < n ? __ldg(Y + (long)i * lsize) : 0.0;
+  // tail factors, ahead of the product (their latency hides behind the loads)
+  const double fl = sqrt((double)(2 * l + 1)) * kInvSqrt4Pi;
+  const double low = wid == 0 ? pow(at.first_x, (double)l) : 1.0;
+  const double high = wid == (n - 1) % W ? pow(at.last_x, (double)(l + 1)) : 1.0;
+  __syncthreads();
+  const int g = lane >> 2, q = lane & 3;
+  const double *G = P.gop + rep.gop_off + (long)l * rows * ld + (long)g * ld + q;
+  for (int r0 = 32 * wid; r0 < rows; r0 += 32 * W) {
+    // two 16-row tiles; beyond the last row the first is repeated, not stored
+    const double *ga[2] = {G + (long)r0 * ld, G + (long)(r0 + 16 < rows ? r0 + 16 : r0) * ld};
+    double acc[2][4][4], a[2][2][4];
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[t][nt][k] = 0.0;
+    auto load = [&](int kk, double(&f)[2][4]) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          f[t][k] = __ldg(ga[t] + (long)(8 * (k & 1)) * ld + kk + 4 * (k >> 1));
+    };
+    auto product = [&](int kk, const double(&f)[2][4]) {
+#pragma unroll
+      for (int nt = 0; nt < 4; ++nt) {
+        const double *x = fs + (kk + q) * kApplyLdf + nt * 8 + g;
+        const double b[2] = {x[0], x[4 * kApplyLdf]};
+        dmma(acc[0][nt], f[0], b);
+        dmma(acc[1][nt], f[1], b);
+      }
+    };
+    // fragments are loaded a step ahead of their products
+    load(0, a[0]);
+    for (int kk = 0; kk < ld; kk += 16) {
+      if (kk + 8 < ld) load(kk + 8, a[1]);
+      product(kk, a[0]);
+      if (kk + 8 >= ld) break;
+      if (kk + 16 < ld) load(kk + 16, a[0]);
+      product(kk + 8, a[1]);
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      if (r0 + 16 * t < rows)
+#pragma unroll
+        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            xs[(r0 + 16 * t + g + 8 * (k >> 1)) * kApplyLdx + nt * 8 + 2 * q + (k & 1)] =
+                acc[t][nt][k];
+  }
+  __syncthreads();
+  if (!live) return;
+  double *spl = P.spl + bat * P.spl_stride + at.spl_off + (long)lm * 4;
+  double *amp = P.amp + bat * P.amp_stride + at.amp_off + lm * 2;
+  for (int i = wid; i < n; i += W) {
+    const double *x = xs + 2 * i * kApplyLdx + lane;
+    const double y0 = x[0], d0 = x[kApplyLdx];
+    if (P.raw_y) {
+      const long o = at.raw_off + (long)lm * n + i;
+      P.raw_y[o] = y0;
+      P.raw_dt[o] = d0;
+    }
+    if (i < n - 1) {
+      const double z = x[2 * kApplyLdx] - y0, d1 = x[3 * kApplyLdx];
+      double2 *cf = reinterpret_cast<double2 *>(spl + (long)i * lsize * 4);
+      cf[0] = make_double2(y0 * fl, d0 * fl);
+      cf[1] = make_double2((3 * z - 2 * d0 - d1) * fl, (-2 * z + d0 + d1) * fl);
+    } else {
+      amp[1] = y0 * high * fl;
+    }
+    if (i == 0) amp[0] = y0 / low * fl;
+  }
 }
 
 // ------------------------------------------------------------------ kinetic
@@ -1639,17 +1784,47 @@ cudaError_t launch_radial_solve(const PoissonDev &P, const RadialOp &op, cudaStr
   const size_t smem = radial_smem_bytes(P.max_nrad, threads);
   if (smem > kMaxSmem || 2 * P.max_lmax + 1 > kRadialThreads || !P.rscr)
     return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(radial_kernel,
+  cudaError_t e = cudaFuncSetAttribute(radial_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int spc = radial_solves_per_cta(P.max_lmax, threads);
   const int groups = (P.nbatch + spc - 1) / spc;
-  radial_kernel<<<dim3(P.nsys, groups), threads, smem, s>>>(P, op);
+  radial_kernel<false><<<dim3(P.nsys, groups), threads, smem, s>>>(P, op, nullptr, 0, nullptr);
+  return cudaGetLastError();
+}
+
+size_t radial_op_tmp_doubles(int nsys, int max_nrad) {
+  return ((size_t)nsys + 1) * max_nrad * max_nrad;
+}
+
+cudaError_t launch_radial_operators(const PoissonDev &P, double *tmp, cudaStream_t s) {
+  if (P.nsys == 0) return cudaSuccess;
+  const int n = P.max_nrad;
+  identity_kernel<<<dim3((n + 127) / 128, n), 128, 0, s>>>(tmp, n);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  constexpr int threads = 32;
+  const size_t smem = radial_smem_bytes(n, threads);
+  if (smem > kMaxSmem) return cudaErrorInvalidValue;
+  e = cudaFuncSetAttribute(radial_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem);
+  if (e != cudaSuccess) return e;
+  radial_kernel<true><<<dim3(P.nsys, (n + threads - 1) / threads), threads, smem, s>>>(
+      P, RadialOp(), tmp, n, tmp + (size_t)n * n);
   return cudaGetLastError();
 }
 
 cudaError_t launch_poisson_radial(const PoissonDev &P, cudaStream_t s) {
-  return launch_radial_solve(P, RadialOp(), s);
+  if (!P.gop) return launch_radial_solve(P, RadialOp(), s);
+  if (P.ngroup == 0) return cudaSuccess;
+  const long tiles = ((long)P.max_group_cols * P.nbatch + kApplyCols - 1) / kApplyCols;
+  const size_t smem = radial_apply_doubles(P.max_nrad) * sizeof(double);
+  if (tiles > 0x7fffffffL || P.ngroup > 65535 || smem > kMaxSmem) return cudaErrorInvalidValue;
+  cudaError_t e = cudaFuncSetAttribute(radial_apply_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  radial_apply_kernel<<<dim3((unsigned)tiles, P.ngroup), kApplyThreads, smem, s>>>(P);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_kinetic_radial(const PoissonDev &P, double scale, cudaStream_t s) {

@@ -27,6 +27,7 @@ struct PoissonAtom {
   int bucket_off;  // [nrad + 1] buckets: 0 left tail, 1 + j interval j, nrad right tail
   int sys_off;     // radial system of (this atom, l) = sys_off + l
   long pair_off;   // this atom's slice of the (atom, point) pair arrays
+  long gop_off;    // radial operators of this radial grid: [lmax + 1][rows][ld]
   long rows_off;   // evaluation rows: [nrad - 1][eval_rows_doubles(lmax)]
   long scr_off;    // radial-solve scratch: [3 nrad][lsize]
 };
@@ -57,6 +58,18 @@ enum : int {
 // pivoting reaches kl + ku above the diagonal, kW stored diagonals.
 constexpr int kKL = 3, kKU = 3, kW = 2 * kKL + kKU + 1;
 
+// Atoms of one radial grid and lmax, at one l: the columns (solve, atom, m) one
+// radial operator serves.
+struct RadialGroup {
+  int first, natom;  // atoms group_atom[first .. first + natom)
+  int l;
+};
+// Radial operators (row 2i: the solution at node i, row 2i + 1 its t-derivative,
+// column j: per unit of f_lm(r_j)), padded with zeros to whole 16 x 8 fragments.
+constexpr int kRadialOpMax = 256;  // largest nrad solved with operators
+__host__ __device__ constexpr int radial_op_rows(int n) { return (2 * n + 15) / 16 * 16; }
+__host__ __device__ constexpr int radial_op_ld(int n) { return (n + 7) / 8 * 8; }
+
 struct PoissonDev {
   int natom = 0, nmol = 0, nsys = 0;
   int max_lmax = 0, max_nrad = 0, max_nang = 0;
@@ -73,6 +86,12 @@ struct PoissonDev {
   double *amp = nullptr;
   double *raw_y = nullptr;
   double *raw_dt = nullptr;
+  // Radial operators, one set per distinct radial grid (null: the Poisson
+  // solves substitute with the LU factors below instead)
+  double *gop = nullptr;
+  RadialGroup *groups = nullptr;
+  int *group_atom = nullptr;
+  int ngroup = 0, max_group_cols = 0;  // largest natom (2 l + 1)
   // LU factors of the radial FEM systems (built once per grid): per system
   // the band [2 nrad][kW], multipliers [2 nrad][3], pivots [2 nrad]; strides
   // use lu_stride = 2 max_nrad rows
@@ -141,7 +160,12 @@ cudaError_t launch_poisson_project(const PoissonDev &P, const double *rho,
                                    cudaStream_t s);
 // Assembles and LU-factors the radial FEM matrices (once per grid).
 cudaError_t launch_poisson_factor(const PoissonDev &P, cudaStream_t s);
-// projected density -> spline tables of the potential (one thread per (solve,
+// Radial operators of P.nsys (radial grid, l) systems into P.gop from their LU
+// factors; tmp holds radial_op_tmp_doubles(nsys, max_nrad).
+size_t radial_op_tmp_doubles(int nsys, int max_nrad);
+cudaError_t launch_radial_operators(const PoissonDev &P, double *tmp, cudaStream_t s);
+// projected density -> spline tables of the potential: a product with the
+// radial operators, or without them substitution (one thread per (solve,
 // l, m) column, one CTA per (atom, l) and group of solves); needs P.rscr.
 cudaError_t launch_poisson_radial(const PoissonDev &P, cudaStream_t s);
 // The same two stages for another radial operator (factors into P.lu, P.lmul,
