@@ -267,7 +267,7 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
     A.mol_npoint = mol_point_off[mol + 1] - mol_point_off[mol];
     plan->max_mol_npoint = std::max(plan->max_mol_npoint, A.mol_npoint);
     A.bucket_off = buckets;
-    buckets += n + 1;
+    buckets += 2 * n;
     A.pair_off = pairs;
     pairs += A.mol_npoint;
     for (int l = 0; l <= lmax; ++l) {
@@ -336,7 +336,7 @@ static int eval_chunk_for(const std::vector<int> &count, const std::vector<Poiss
   long pairs = 0, buckets = 0;
   for (const PoissonAtom &a : ha)
     for (int b = 1; b < a.nrad; ++b) {
-      const int c = count[a.bucket_off + b];
+      const int c = count[a.bucket_off + b] + count[a.bucket_off + a.nrad + b];
       if (c > 0) {
         pairs += c;
         ++buckets;
@@ -356,7 +356,7 @@ int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const 
   PoissonDev &d = plan->d;
   const std::vector<PoissonAtom> &ha = plan->h_atoms;
   int nb = 0;
-  for (auto &a : ha) nb += a.nrad + 1;
+  for (auto &a : ha) nb += 2 * a.nrad;
   // buffers of an earlier geometry or mask are reused; the pairs' buckets are
   // only needed here and lie in pair_v, which the next evaluation overwrites
   NAPMO_TRY_CUDA(plan->pair_v.reserve(d.npair), "pair lists");
@@ -377,7 +377,7 @@ int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const 
   chunk = eval_chunk_for(hc, ha);
   for (int a = 0; a < (int)ha.size(); ++a) {
     int acc = 0;
-    for (int b = 0; b <= ha[a].nrad; ++b) {
+    for (int b = 0; b < 2 * ha[a].nrad; ++b) {
       const int k = ha[a].bucket_off + b;
       start[k] = acc;
       for (int c = 0; c < hc[k]; c += chunk)
@@ -397,10 +397,10 @@ int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const 
   // interior buckets first, the tails after them: the evaluation runs them as
   // two kernels, each with the code of its own region only
   std::stable_partition(hitems.begin(), hitems.end(), [&](const EvalItem &it) {
-    return it.bucket > 0 && it.bucket < ha[it.atom].nrad;
+    return it.bucket > 0 && it.bucket != ha[it.atom].nrad;
   });
   nitems_in = 0;
-  for (const EvalItem &it : hitems) nitems_in += (it.bucket > 0 && it.bucket < ha[it.atom].nrad);
+  for (const EvalItem &it : hitems) nitems_in += (it.bucket > 0 && it.bucket != ha[it.atom].nrad);
   NAPMO_TRY_CUDA(items.reserve(hitems.size()), "pair lists");
   NAPMO_TRY_CUDA(cudaMemcpyAsync(items.p, hitems.data(), hitems.size() * sizeof(EvalItem),
                                  cudaMemcpyHostToDevice, s),

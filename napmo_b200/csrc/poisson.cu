@@ -1123,9 +1123,12 @@ evaluate_kernel(PoissonDev P, int npoint, const double *__restrict__ gx,
 // Bucket of the pair (atom A, point p): 0 below the first radial point, 1 + j
 // inside spline interval j, nrad above the last point -- the same region and
 // interval test as the spline evaluation of the reference
-// (src/horton/cubic_spline.cpp:147-181).
-__device__ __forceinline__ int pair_bucket(const PoissonAtom &at, double px, double py,
+// (src/horton/cubic_spline.cpp:147-181) -- and nrad + 1 + j for the atom's own
+// points of shell j < nrad - 1, which lie on node j of the spline.
+__device__ __forceinline__ int pair_bucket(const PoissonAtom &at, int p, double px, double py,
                                            double pz) {
+  const int own = p - at.point_off;
+  if (own >= 0 && own < (at.nrad - 1) * at.nang) return at.nrad + 1 + own / at.nang;
   const double dx = px - at.cx, dy = py - at.cy, dz = pz - at.cz;
   const double d = sqrt(dx * dx + dy * dy + dz * dz);
   if (d < at.first_x) return 0;
@@ -1153,7 +1156,7 @@ __global__ void pair_bucket_kernel(PoissonDev P, const double *__restrict__ gx,
   int b = -1;
   if (in) {
     const int p = at.mol_point_start + q;
-    if (!keep || keep[p]) b = pair_bucket(at, gx[p], gy[p], gz[p]);  // -1: screened out
+    if (!keep || keep[p]) b = pair_bucket(at, p, gx[p], gy[p], gz[p]);  // -1: screened out
     bucket_of[at.pair_off + q] = b;
   }
   const unsigned group = __match_any_sync(0xffffffffu, b);
@@ -1185,9 +1188,9 @@ __global__ void pair_scatter_kernel(PoissonDev P, const double *__restrict__ gx,
     const long slot = at.pair_off + base + lanes_below(group);
     const int p = at.mol_point_start + q;
     P.pairs[slot] = p;
-    if (b > 0 && b < at.nrad) {  // interior: the evaluation's u and 1/d
+    if (b > 0 && b != at.nrad) {  // interior: the evaluation's u and 1/d
       const double d = pair_distance(at, gx, gy, gz, p);
-      P.pair_u[slot] = make_double2(rt_inv(at.rt, d) - (b - 1), 1.0 / d);
+      P.pair_u[slot] = make_double2(b < at.nrad ? rt_inv(at.rt, d) - (b - 1) : 0.0, 1.0 / d);
     }
   }
 }
@@ -1235,7 +1238,7 @@ __host__ __device__ constexpr int eval_rows(int lmax) { return eval_family(lmax,
 
 // One family: columns m0 and m0 + 1, rows n < nodd of both and row nodd of m0
 // alone (m0 + 1 has its last term one row before).
-template <int NP, bool SIN>
+template <int NP, bool SIN, bool NODE>
 __device__ __forceinline__ void family_sums(const double *row, int nodd, const double *rec,
                                             double start, const double *z, const double *u,
                                             double *ec, double *es, double *oc, double *os) {
@@ -1245,6 +1248,13 @@ __device__ __forceinline__ void family_sums(const double *row, int nodd, const d
   auto add = [&](const double *c, auto &...s) {
     constexpr int G = sizeof...(s);
     double *const sp[G] = {s...};
+    if constexpr (NODE) {  // u = 0: the cubics' first coefficients
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int j = 0; j < NP; ++j) sp[g][j] = fma(c[4 * g], b[j], sp[g][j]);
+      return;
+    }
     double2 lo[G], hi[G];
     double t[G][NP];
 #pragma unroll
@@ -1297,13 +1307,16 @@ __device__ __forceinline__ void family_sums(const double *row, int nodd, const d
     add(row, ec);
 }
 
-template <int NP>
+// NODE: pairs on the interval's first node (an atom and its own points), where
+// the cubics are their first coefficients: 440 operations per pair at lmax 14
+// instead of 1100 (35 solves of HCN, 1 of 3 pairs: 850 -> 734 us).
+template <int NP, bool NODE>
 __device__ __forceinline__ void interior_values(const double *cf, int L, const double *x,
                                                 const double *y, const double *z,
                                                 const double *u, double *v) {
   double cm[NP], sm[NP], ec[NP], es[NP], oc[NP], os[NP];
   const double *rec = c_rec_a + kMaxLmax + 1;  // A at [l = m0 + 1][m0]
-  family_sums<NP, false>(cf, L, rec, 1.0, z, u, ec, es, oc, os);
+  family_sums<NP, false, NODE>(cf, L, rec, 1.0, z, u, ec, es, oc, os);
 #pragma unroll
   for (int j = 0; j < NP; ++j) {
     cm[j] = x[j];
@@ -1322,7 +1335,7 @@ __device__ __forceinline__ void interior_values(const double *cf, int L, const d
   for (int m0 = 2; m0 <= L; m0 += 2) {
     cf += kEvalRow * (L + 3 - m0);  // past the L + 1 - (m0 - 2) rows of the last family
     rec += 2 * (kMaxLmax + 1) + 2;
-    family_sums<NP, true>(cf, L - m0, rec, c_rec_start[m0], z, u, ec, es, oc, os);
+    family_sums<NP, true, NODE>(cf, L - m0, rec, c_rec_start[m0], z, u, ec, es, oc, os);
     rotate();
 #pragma unroll
     for (int j = 0; j < NP; ++j) v[j] = fma(cm[j], ec[j], fma(sm[j], es[j], v[j]));
@@ -1504,21 +1517,29 @@ template <int LMAX, bool TAILS, bool BATCH>
 // Four 128-thread CTAs per SM (128 registers): 16 warps with eight independent
 // products each.  Measured at C12H26: two pairs per thread at 64 registers
 // 3.74 ms, three at 80 3.77 ms, four at 96 3.87 ms and at 128 3.55 ms.
-__global__ void __launch_bounds__(kEvalChunkMax / kEvalPerThread, 4)
+// The tails take one pair per thread: few CTAs, so the length of a thread's
+// chain is their time (C12H26: 24 us instead of 44 with four; in one launch
+// with the interior they cost its code more than their time, C20H42 4.59 ->
+// 5.00 ms).
+__global__ void __launch_bounds__(kEvalChunkMax / (TAILS ? 1 : kEvalPerThread), TAILS ? 1 : 4)
 eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
                   const double *__restrict__ gy, const double *__restrict__ gz) {
   extern __shared__ double cf[];
+  constexpr int NP = TAILS ? 1 : kEvalPerThread;
   const EvalItem it = P.items[blockIdx.x + (TAILS ? P.nitems_inner : 0)];
   const PoissonAtom &at = P.atoms[it.atom];
   const int lmaxA = at.lmax;
   const int lsize = (lmaxA + 1) * (lmaxA + 1);
-  const int region = TAILS ? (it.bucket == 0 ? 1 : 2) : 0;
+  // an own-shell bucket nrad + 1 + j reads interval j's rows
+  const bool node = !TAILS && it.bucket > at.nrad;
+  const int bucket = node ? it.bucket - at.nrad : it.bucket;
+  const int region = TAILS ? (bucket == 0 ? 1 : 2) : 0;
   const long bat = BATCH ? (long)blockIdx.y : 0;  // solve of a batch
   // l-blocks kept for this bucket (all unless a truncation tolerance is set)
-  const int lcut = P.lcut ? P.lcut[bat * P.lcut_stride + at.bucket_off + it.bucket] : lmaxA;
+  const int lcut = P.lcut ? P.lcut[bat * P.lcut_stride + at.bucket_off + bucket] : lmaxA;
   if (region == 0) {  // 16-byte copies in flight while the pairs are read
     const double *src = P.rows + bat * P.rows_stride + at.rows_off +
-                        (long)(it.bucket - 1) * kEvalRow * eval_rows(lmaxA);
+                        (long)(bucket - 1) * kEvalRow * eval_rows(lmaxA);
     for (int e = threadIdx.x; e < kEvalRow / 2 * eval_rows(lcut); e += blockDim.x)
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
                        (unsigned)__cvta_generic_to_shared(cf + 2 * e)),
@@ -1532,11 +1553,11 @@ eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
   // thread t evaluates the pairs t + j blockDim.x of the item (an absent one
   // repeats the item's first and is not stored)
   const int t = threadIdx.x;
-  int pidx[kEvalPerThread];
-  double x[kEvalPerThread], y[kEvalPerThread], z[kEvalPerThread], d[kEvalPerThread],
-      inv[kEvalPerThread], u[kEvalPerThread], v[kEvalPerThread];
+  int pidx[NP];
+  double x[NP], y[NP], z[NP], d[NP],
+      inv[NP], u[NP], v[NP];
 #pragma unroll
-  for (int j = 0; j < kEvalPerThread; ++j) {
+  for (int j = 0; j < NP; ++j) {
     const int e = t + j * (int)blockDim.x;
     const long slot = at.pair_off + it.start + (e < it.count ? e : 0);
     pidx[j] = P.pairs[slot];
@@ -1559,14 +1580,16 @@ eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
   if (!TAILS) asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
   if (t >= it.count) return;
-  if (!TAILS)
-    interior_values<kEvalPerThread>(cf, lcut, x, y, z, u, v);
+  if (node)
+    interior_values<NP, true>(cf, lcut, x, y, z, u, v);
+  else if (!TAILS)
+    interior_values<NP, false>(cf, lcut, x, y, z, u, v);
   else if (region == 1)
-    tail_values<LMAX, 1, kEvalPerThread>(cf, lcut, x, y, z, d, inv, v);
+    tail_values<LMAX, 1, NP>(cf, lcut, x, y, z, d, inv, v);
   else
-    tail_values<LMAX, 2, kEvalPerThread>(cf, lcut, x, y, z, d, inv, v);
+    tail_values<LMAX, 2, NP>(cf, lcut, x, y, z, d, inv, v);
 #pragma unroll
-  for (int j = 0; j < kEvalPerThread; ++j) {
+  for (int j = 0; j < NP; ++j) {
     const int e = t + j * (int)blockDim.x;
     if (e < it.count)
       P.pair_v[bat * P.pairv_stride + at.pair_off + (pidx[j] - at.mol_point_start)] = v[j];
@@ -1615,7 +1638,7 @@ cudaError_t launch_eval_l(const PoissonDev &P, int npoint, const double *x,
     const size_t smem = (size_t)kEvalRow * eval_rows(L) * sizeof(double);
     const size_t smem_tail = (size_t)(L + 1) * (L + 1) * sizeof(double);
     const dim3 gin(P.nitems_inner, P.nbatch), gtail(P.nitems - P.nitems_inner, P.nbatch);
-    const int kT = P.eval_chunk / kEvalPerThread;
+    const int kT = P.eval_chunk / kEvalPerThread, kTail = P.eval_chunk;
     if (P.nitems_inner > 0) {
       if (P.nbatch > 1)
         eval_pairs_kernel<L, false, true><<<gin, kT, smem, s>>>(P, x, y, z);
@@ -1624,9 +1647,9 @@ cudaError_t launch_eval_l(const PoissonDev &P, int npoint, const double *x,
     }
     if (P.nitems > P.nitems_inner) {
       if (P.nbatch > 1)
-        eval_pairs_kernel<L, true, true><<<gtail, kT, smem_tail, s>>>(P, x, y, z);
+        eval_pairs_kernel<L, true, true><<<gtail, kTail, smem_tail, s>>>(P, x, y, z);
       else
-        eval_pairs_kernel<L, true, false><<<gtail, kT, smem_tail, s>>>(P, x, y, z);
+        eval_pairs_kernel<L, true, false><<<gtail, kTail, smem_tail, s>>>(P, x, y, z);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;

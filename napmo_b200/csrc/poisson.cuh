@@ -24,7 +24,8 @@ struct PoissonAtom {
   int amp_off;    // [lsize][2] left / right extrapolation amplitudes (scaled)
   int raw_off;    // [lsize][nrad] solution values y and t-derivatives dt
   int mol_point_start, mol_npoint;  // points of this atom's molecule
-  int bucket_off;  // [nrad + 1] buckets: 0 left tail, 1 + j interval j, nrad right tail
+  int bucket_off;  // [2 nrad] buckets: 0 left tail, 1 + j interval j, nrad right tail,
+                   // nrad + 1 + j own points on node j < nrad - 1
   int sys_off;     // radial system of (this atom, l) = sys_off + l
   long pair_off;   // this atom's slice of the (atom, point) pair arrays
   long gop_off;    // radial operators of this radial grid: [lmax + 1][rows][ld]
