@@ -59,12 +59,15 @@ struct PoissonPlan {
   DevBuf<int> bucket_count;  // pair-list construction
   bool moved = false;        // the grid's centres moved: centres and pair lists are stale
   // pair lists of the points kept by a screening mask (built for the last
-  // mask used; the mask is owned by the caller's int8 plan)
-  DevBuf<int> pairs_s;
-  DevBuf<double2> pair_u_s;
-  DevBuf<EvalItem> items_s;
-  int nitems_s = 0, nitems_in_s = 0, chunk_s = kEvalChunk;
-  unsigned long long screen_key = 0;  // serial of the mask's int8 plan (0: none)
+  // mask used; the mask is owned by the caller's int8 plan): [0] for truncated
+  // solves, [1] with node buckets for the others
+  struct Screened {
+    DevBuf<int> pairs;
+    DevBuf<double2> pair_u;
+    DevBuf<EvalItem> items;
+    int nitems = 0, nitems_in = 0, chunk = kEvalChunk;
+    unsigned long long key = 0;  // serial of the mask's int8 plan (0: none)
+  } screened[2];
   // Becke-Dickson workspace (source, shell averages, LU factors), kept
   // between calls: an allocation per call would return to the driver at
   // every synchronisation of the caller's loop
@@ -350,7 +353,7 @@ static int eval_chunk_for(const std::vector<int> &count, const std::vector<Poiss
 // items; with `keep` only the points whose flag is set.  Built once per grid
 // (and once per screening mask); about 12 bytes per pair.  Synchronises `s`.
 int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const double *z,
-                     const int *keep, DevBuf<int> &pairs, DevBuf<double2> &pair_u,
+                     const int *keep, bool nodes, DevBuf<int> &pairs, DevBuf<double2> &pair_u,
                      DevBuf<EvalItem> &items, int &nitems, int &nitems_in, int &chunk,
                      cudaStream_t s) {
   PoissonDev &d = plan->d;
@@ -365,7 +368,8 @@ int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const 
   int *const bucket_of = reinterpret_cast<int *>(plan->pair_v.p);
   int *const count = plan->bucket_count.p;
   NAPMO_TRY_CUDA(cudaMemsetAsync(count, 0, nb * sizeof(int), s), "pair lists");
-  NAPMO_TRY_CUDA(launch_pair_buckets(d, plan->max_mol_npoint, x, y, z, keep, bucket_of, count, s),
+  NAPMO_TRY_CUDA(launch_pair_buckets(d, plan->max_mol_npoint, x, y, z, keep, nodes, bucket_of,
+                                     count, s),
                  "pair buckets");
   std::vector<int> hc(nb);
   NAPMO_TRY_CUDA(cudaMemcpyAsync(hc.data(), count, nb * sizeof(int), cudaMemcpyDeviceToHost, s),
@@ -411,25 +415,43 @@ int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const 
   return kOk;
 }
 
-// Points the evaluation runs on: all (keep null) or the screened ones.
+// Points the evaluation runs on: all (keep null) or the screened ones, whose
+// lists depend on whether the solves truncate (tol > 0, see pair_bucket).  The
+// two forms agree to rounding and within tol: a capturing stream, where nothing
+// can be built, takes the other if that is what there is.
 static int select_pair_lists(PoissonPlan *p, BeckeGrid *g, const int *keep,
-                             unsigned long long key, cudaStream_t s) {
+                             unsigned long long key, double tol, cudaStream_t s) {
   PoissonDev &d = p->d;
-  if (keep && key != p->screen_key) {
-    p->screen_key = 0;
-    const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, keep, p->pairs_s,
-                                    p->pair_u_s, p->items_s, p->nitems_s, p->nitems_in_s,
-                                    p->chunk_s, s);
-    if (st) return st;
-    p->screen_key = key;
-  }
   d.keep = keep;
-  d.pairs = keep ? p->pairs_s.p : p->pairs.p;
-  d.pair_u = keep ? p->pair_u_s.p : p->pair_u.p;
-  d.items = keep ? p->items_s.p : p->items.p;
-  d.nitems = keep ? p->nitems_s : p->nitems;
-  d.nitems_inner = keep ? p->nitems_in_s : p->nitems_in;
-  d.eval_chunk = keep ? p->chunk_s : p->chunk;
+  if (!keep) {
+    d.pairs = p->pairs.p;
+    d.pair_u = p->pair_u.p;
+    d.items = p->items.p;
+    d.nitems = p->nitems;
+    d.nitems_inner = p->nitems_in;
+    d.eval_chunk = p->chunk;
+    return kOk;
+  }
+  bool nodes = !(tol > 0.0);
+  if (key != p->screened[nodes].key && key == p->screened[!nodes].key) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    NAPMO_TRY_CUDA(cudaStreamIsCapturing(s, &c), "pair lists");
+    if (c != cudaStreamCaptureStatusNone) nodes = !nodes;
+  }
+  PoissonPlan::Screened &l = p->screened[nodes];
+  if (key != l.key) {
+    l.key = 0;
+    const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, keep, nodes, l.pairs,
+                                    l.pair_u, l.items, l.nitems, l.nitems_in, l.chunk, s);
+    if (st) return st;
+    l.key = key;
+  }
+  d.pairs = l.pairs.p;
+  d.pair_u = l.pair_u.p;
+  d.items = l.items.p;
+  d.nitems = l.nitems;
+  d.nitems_inner = l.nitems_in;
+  d.eval_chunk = l.chunk;
   return kOk;
 }
 
@@ -449,8 +471,8 @@ static int move_poisson_plan(BeckeGrid *g, PoissonPlan *p, cudaStream_t s) {
                                  p->h_atoms.size() * sizeof(PoissonAtom),
                                  cudaMemcpyHostToDevice, s),
                  "move atoms");
-  p->screen_key = 0;
-  const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, p->pairs, p->pair_u,
+  p->screened[0].key = p->screened[1].key = 0;
+  const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, true, p->pairs, p->pair_u,
                                   p->items, p->nitems, p->nitems_in, p->chunk, s);
   if (st) return st;
   d.keep = nullptr;
@@ -500,7 +522,7 @@ int grid_poisson_plan(BeckeGrid *g, int lmax, cudaStream_t s, PoissonPlan **out)
     delete p;
     return st;
   }
-  st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, p->pairs, p->pair_u,
+  st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, true, p->pairs, p->pair_u,
                         p->items, p->nitems, p->nitems_in, p->chunk, s);
   if (st != kOk) {
     delete p;
@@ -572,7 +594,7 @@ int grid_concat(const std::vector<BeckeGrid *> &grids, const std::vector<int> &l
   for (auto &L : g->layout) atoms.push_back(&L);
   int st = build_poisson_plan(atoms, lm, mol_atom_off, o, s, p);
   if (st != kOk) return st;
-  st = build_pair_lists(p, d.x, d.y, d.z, nullptr, p->pairs, p->pair_u, p->items, p->nitems,
+  st = build_pair_lists(p, d.x, d.y, d.z, nullptr, true, p->pairs, p->pair_u, p->items, p->nitems,
                         p->nitems_in, p->chunk, s);
   if (st != kOk) return st;
   p->d.items = p->items.p;
@@ -591,7 +613,7 @@ void grid_free(BeckeGrid *g) { delete g; }
 int run_poisson(BeckeGrid *g, PoissonPlan *p, const double *rho_dev, double *v_dev,
                 bool accumulate, cudaStream_t s, double tol, const int *keep,
                 unsigned long long key) {
-  int st = select_pair_lists(p, g, keep, key, s);
+  int st = select_pair_lists(p, g, keep, key, tol, s);
   if (st) return st;
   p->d.eval_tol = tol;
   p->d.lcut = tol > 0.0 ? p->lcut.p : nullptr;
@@ -611,7 +633,7 @@ static int operator_dev(BeckeGrid *g, int lmax, cudaStream_t s, PoissonDev *out,
   int st = grid_poisson_plan(g, lmax, s, &p);
   if (st) return st;
   if (plan) *plan = p;
-  st = select_pair_lists(p, g, nullptr, 0, s);
+  st = select_pair_lists(p, g, nullptr, 0, 0.0, s);
   if (st) return st;
   *out = p->d;
   out->eval_tol = 0.0;
@@ -671,7 +693,7 @@ int run_poisson_many(BeckeGrid *g, PoissonPlan *p, int k, const double *rho_dev,
                      double *v_dev, cudaStream_t s, double tol, const int *keep,
                      unsigned long long key) {
   if (k <= 0) return kOk;
-  int st = select_pair_lists(p, g, keep, key, s);
+  int st = select_pair_lists(p, g, keep, key, tol, s);
   if (st) return st;
   const PoissonDev &d = p->d;
   const size_t nscr = d.gop ? 0 : p->rscr.n;  // the operators need no scratch

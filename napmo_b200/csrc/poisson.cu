@@ -134,6 +134,7 @@ __device__ __forceinline__ double rt_inv(const RTParams &rt, double r) {
 // kProjStages - 1 chunks ahead of its products.
 constexpr int kProjTile = 64, kProjK = 16, kProjThreads = 128, kProjStages = 3;
 constexpr int kProjLda = kProjK + 4, kProjLdb = kProjTile + 4;
+static_assert(kProjThreads == 2 * kProjTile, "one thread per row and column factor");
 constexpr int kProjPer = kProjTile * kProjK / kProjThreads;  // copies per thread per chunk
 constexpr size_t kProjStageDoubles = kProjTile * kProjLda + kProjK * kProjLdb;
 
@@ -159,6 +160,10 @@ __device__ __forceinline__ void proj_copy8(double *dst, const double *src, bool 
 
 __global__ void __launch_bounds__(kProjThreads, 3) project_kernel(PoissonDev P) {
   extern __shared__ __align__(16) double psm[];
+  // factors of the tile's columns and rows, formed while the first copies fly:
+  // a root and a division per element at the end took longer than the products
+  // of a small atom (H2O 50 x 110 15 -> 9.5 us)
+  __shared__ double col_fac[kProjTile], row_inv[kProjTile];
   const int bat = blockIdx.z / P.natom;  // solve of a batch
   const PoissonAtom at = P.atoms[blockIdx.z - bat * P.natom];
   const double *g = P.pg + bat * P.pg_stride;
@@ -206,6 +211,13 @@ __global__ void __launch_bounds__(kProjThreads, 3) project_kernel(PoissonDev P) 
     if (c < nchunk) issue(c);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
+  if (t < kProjTile) {
+    const int l = (int)sqrtf((float)(lm0 + t));  // exact: below 2^23
+    col_fac[t] = sqrt(4.0 * M_PI * (2.0 * l + 1));
+  } else {
+    const int sh = s0 + t - kProjTile;
+    row_inv[t - kProjTile] = sh < nrad ? 1.0 / P.rad[at.rad_off + kRadSigma * nrad + sh] : 0.0;
+  }
   for (int c = 0; c < nchunk; ++c) {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kProjStages - 2) : "memory");
     __syncthreads();  // chunk c is in for every thread; stage (c - 1) is free
@@ -237,22 +249,20 @@ __global__ void __launch_bounds__(kProjThreads, 3) project_kernel(PoissonDev P) 
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  const double *sigma = P.rad + at.rad_off + kRadSigma * nrad;
 #pragma unroll
   for (int nt = 0; nt < 4; ++nt) {
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const int lm = lm0 + wc + nt * 8 + 2 * q + c;
+      const int col = wc + nt * 8 + 2 * q + c, lm = lm0 + col;
       if (lm >= lsize) continue;
-      const int l = (int)sqrt((double)lm + 0.5);
-      const double fac = sqrt(4.0 * M_PI * (2.0 * l + 1));
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int sh = s0 + wr + mt * 16 + gq + 8 * h;
-          if (sh < nrad)
-            proj[at.proj_off + (long)sh * lsize + lm] = acc[mt][nt][2 * h + c] / sigma[sh] * fac;
+          const int row = wr + mt * 16 + gq + 8 * h;
+          if (s0 + row < nrad)
+            proj[at.proj_off + (long)(s0 + row) * lsize + lm] =
+                acc[mt][nt][2 * h + c] * row_inv[row] * col_fac[col];
         }
       }
     }
@@ -1124,11 +1134,13 @@ evaluate_kernel(PoissonDev P, int npoint, const double *__restrict__ gx,
 // inside spline interval j, nrad above the last point -- the same region and
 // interval test as the spline evaluation of the reference
 // (src/horton/cubic_spline.cpp:147-181) -- and nrad + 1 + j for the atom's own
-// points of shell j < nrad - 1, which lie on node j of the spline.
+// points of shell j < nrad - 1, which lie on node j of the spline (not in lists
+// for truncated solves, `nodes` false: those truncate by interval, and rounding
+// puts a node into either of its two).
 __device__ __forceinline__ int pair_bucket(const PoissonAtom &at, int p, double px, double py,
-                                           double pz) {
+                                           double pz, bool nodes) {
   const int own = p - at.point_off;
-  if (own >= 0 && own < (at.nrad - 1) * at.nang) return at.nrad + 1 + own / at.nang;
+  if (nodes && own >= 0 && own < (at.nrad - 1) * at.nang) return at.nrad + 1 + own / at.nang;
   const double dx = px - at.cx, dy = py - at.cy, dz = pz - at.cz;
   const double d = sqrt(dx * dx + dy * dy + dz * dz);
   if (d < at.first_x) return 0;
@@ -1149,14 +1161,15 @@ __device__ __forceinline__ int lanes_below(unsigned m) {
 __global__ void pair_bucket_kernel(PoissonDev P, const double *__restrict__ gx,
                                    const double *__restrict__ gy,
                                    const double *__restrict__ gz, const int *__restrict__ keep,
-                                   int *__restrict__ bucket_of, int *__restrict__ count) {
+                                   bool nodes, int *__restrict__ bucket_of,
+                                   int *__restrict__ count) {
   const PoissonAtom &at = P.atoms[blockIdx.y];
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = q < at.mol_npoint;
   int b = -1;
   if (in) {
     const int p = at.mol_point_start + q;
-    if (!keep || keep[p]) b = pair_bucket(at, p, gx[p], gy[p], gz[p]);  // -1: screened out
+    if (!keep || keep[p]) b = pair_bucket(at, p, gx[p], gy[p], gz[p], nodes);  // -1: screened out
     bucket_of[at.pair_off + q] = b;
   }
   const unsigned group = __match_any_sync(0xffffffffu, b);
@@ -1873,10 +1886,10 @@ cudaError_t launch_shell_average(const PoissonDev &P, const double *f, const dou
 }
 
 cudaError_t launch_pair_buckets(const PoissonDev &P, int max_mol_npoint, const double *x,
-                                const double *y, const double *z, const int *keep,
+                                const double *y, const double *z, const int *keep, bool nodes,
                                 int *bucket_of, int *count, cudaStream_t s) {
   dim3 grid((max_mol_npoint + 255) / 256, P.natom);
-  pair_bucket_kernel<<<grid, 256, 0, s>>>(P, x, y, z, keep, bucket_of, count);
+  pair_bucket_kernel<<<grid, 256, 0, s>>>(P, x, y, z, keep, nodes, bucket_of, count);
   return cudaGetLastError();
 }
 

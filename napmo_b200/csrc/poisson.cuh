@@ -189,7 +189,7 @@ cudaError_t launch_shell_average(const PoissonDev &P, const double *f, const dou
 // writes its own slot of pair_v).
 // With keep non-null, points whose flag is 0 get no pair (bucket -1).
 cudaError_t launch_pair_buckets(const PoissonDev &P, int max_mol_npoint, const double *x,
-                                const double *y, const double *z, const int *keep,
+                                const double *y, const double *z, const int *keep, bool nodes,
                                 int *bucket_of, int *count, cudaStream_t s);
 // The scatter also stores, for the pairs of interior buckets, the spline
 // interval coordinate u = rt_inv(|p - A|) - j and 1 / |p - A| in P.pair_u
