@@ -1085,10 +1085,11 @@ def main():
     fbld.set_precision(headline)
     t_dev = t_tc if headline == 'int8x4' else t_f64
     clocks = clocks_tc if headline == 'int8x4' else clocks_f64
-    # kernels per build: density (FP64: 1; int8: slice D + density), Poisson
-    # (project, radial, pair evaluation, pair reduce), weights, quadrature
-    # (FP64: GEMM + reduce; int8: slice wv phi + GEMM + reduce)
-    launches_per_build = 9 if headline == 'int8x4' else 8
+    # kernels per build: density (FP64: 1; int8: symmetrise D + slice D + density),
+    # Poisson (weighted density, project, radial product, rows, interior and tail
+    # evaluation, pair reduce), weights, quadrature (FP64: GEMM + reduce; int8:
+    # group scales + slice wv phi + GEMM + reduce)
+    launches_per_build = 15 if headline == 'int8x4' else 11
     mixed = {'builds_per_s': world * args.steps / t_tc, 'ms_per_build': t_tc / args.steps * 1e3,
              'energy_error_eh': dE, 'max_abs_dF': float((F - F64).abs().max()),
              'speedup_vs_fp64': t_f64 / t_tc, 'tc_status': tc_err,
@@ -1179,13 +1180,14 @@ def main():
         if dom == 'poisson':
             # potential evaluation dominates: FP64 ALU bound.  Algorithmic count:
             # 20 flops per (atom, point, lm) as nAPMO evaluates it; the kernel
-            # executes about 10.5 L(L+1) + 11 (L+1) + 3 L + 20 flops per
-            # (atom, point): per (l, m > 0) the rescaled recursion (3), the two
-            # products with cos/sin (2) and two 4-coefficient terms (16).
+            # executes about 8 (L+1)^2 + 3 (h+1)(L-h) + 10 L flops per (atom,
+            # point), h = L // 2: a cubic and its sum per (l, m) (8), the
+            # recursion shared by two columns (3 per step), cos/sin per m (10).
             natom = len(atoms)
             lsize = (lmax + 1) ** 2
             flops_alg = 20.0 * natom * lsize * N
-            flops_exec = (10.5 * lmax * (lmax + 1) + 11.0 * (lmax + 1) + 3.0 * lmax + 20.0) * natom * N
+            h = lmax // 2
+            flops_exec = (8.0 * lsize + 3.0 * (h + 1) * (lmax - h) + 10.0 * lmax) * natom * N
             achieved = flops_alg / td / 1e12
             peak = fp64
             bound = 'fp64'
@@ -1193,7 +1195,7 @@ def main():
                            'HBM/bf16 only); stage = projection + radial + evaluation + reduce (FP64 '
                            'mode, untruncated), the evaluation kernel is 94 % of it (launch list). '
                            'frac exceeds 1 because the algorithmic count is 20 flops per (pair, lm) '
-                           'while the kernel executes about 10.5: see issued')
+                           'while the kernel executes about 9.4: see issued')
             issued = {'executed_fp64_tflops': flops_exec / td / 1e12,
                       'frac_executed': flops_exec / td / 1e12 / fp64}
             kernel_name = 'poisson(eval_pairs dominant)'
