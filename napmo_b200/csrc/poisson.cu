@@ -797,9 +797,10 @@ __global__ void identity_kernel(double *a, int ld) {
 
 // Radial solve by operator: X = G_l F for the columns (solve, atom, m) of one
 // group (atoms of one radial grid and lmax), G_l [2 nrad][nrad].  CTA = (group,
-// 32 columns): F is staged in shared memory, a warp forms 32 rows at a time FP64 tensor pipe with G's fragments read straight from L2 (each is used once per
-// CTA), and X, staged in shared memory, leaves as the cubic of
-// every interval and the tail amplitudes.  Every column's sums run over the
+// 32 columns): F is staged in shared memory, a warp forms 32 rows at a time on
+// the FP64 tensor pipe with G's fragments read straight from L2 (each is used
+// once per CTA), and X, staged in shared memory, leaves as the cubic of every
+// interval and the tail amplitudes.  Every column's sums run over the
 // radial points in order, whatever the batch.
 // Substituting instead costs 6 nrad dependent steps of some 180 ns with one
 // warp per (atom, l); this costs 4 nrad^2 operations per column, all
