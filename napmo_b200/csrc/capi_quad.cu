@@ -234,6 +234,7 @@ struct StageBatch {
   DevBuf<double> rho, v, wv;         // concatenated
   DevBuf<int> keep;                  // concatenated screening flags (screened plans)
   unsigned long long keep_key = 0;
+  DevBuf<double> fold;               // folded density matrices (FP64 plans)
   DevBuf<DensBatchArg> dargs;
   DevBuf<QuadBatchArg> qargs;
   DevBuf<WeightBatchArg> wargs;
@@ -315,14 +316,17 @@ int stage_batch_new(const std::vector<FockPlan *> &plans, const std::vector<doub
   std::vector<QuadBatchArg> qa(nmol);
   std::vector<WeightBatchArg> wa(nmol);
   std::vector<int4> di, qi;
+  size_t fold = 0;
+  for (FockPlan *p : plans) fold += density_fold_doubles(p->n);
+  NAPMO_TRY_CUDA(b->fold.alloc(b->mode == 0 ? std::max<size_t>(fold, 1) : 1), "alloc batch");
+  fold = 0;
   for (int m = 0; m < nmol; ++m) {
     FockPlan *p = plans[m];
     const int N = p->grid->size;
     const bool scr = p->fp64_screen > 0.0;
     da[m] = DensBatchArg{p->phi.p, p->ld, D[m], b->rho.p + b->off[m],
-                         scr ? p->keep64.p : nullptr, p->n, N,
-                         (p->n % 2 == 0 && reinterpret_cast<uintptr_t>(D[m]) % 16 == 0) ? 1 : 0,
-                         0};
+                         scr ? p->keep64.p : nullptr, b->fold.p + fold, p->n, N};
+    fold += density_fold_doubles(p->n);
     std::vector<int> groups, blocks;
     if (scr) {
       groups.resize(p->ngroups64);
@@ -399,7 +403,9 @@ int stage_batch_build(StageBatch *b, cudaStream_t s) {
     NAPMO_TRY_CUDA(launch_combine_weights_batch(b->wargs.p, nmol, b->q, s), "weights");
     return int8_batch_quadrature(b->i8, s);
   }
-  NAPMO_TRY_CUDA(launch_density_batch(b->dargs.p, stage_queue(b, 0), b->grid_d, s), "density");
+  NAPMO_TRY_CUDA(launch_density_batch(b->dargs.p, b->fold.n > 1 ? nmol : 0, stage_queue(b, 0),
+                                      b->grid_d, s),
+                 "density");
   int e = run_poisson(b->cat, b->cat->poisson, b->rho.p, b->v.p, false, s, b->tol,
                       b->keep.p, b->keep_key);
   if (e) return e;
@@ -422,7 +428,7 @@ int stage_batch_queue_selftest(StageBatch *b, unsigned long long timeout_ns, cud
   BatchQueue q = stage_queue(b, 0);
   q.posted = never.p;
   q.timeout_ns = timeout_ns;
-  NAPMO_TRY_CUDA(launch_density_batch(b->dargs.p, q, b->grid_d, s), "self-test");
+  NAPMO_TRY_CUDA(launch_density_batch(b->dargs.p, 0, q, b->grid_d, s), "self-test");
   NAPMO_TRY_CUDA(cudaMemcpyAsync(status, b->status.p, sizeof(int), cudaMemcpyDeviceToHost, s),
                  "self-test");
   NAPMO_TRY_CUDA(cudaMemsetAsync(b->status.p, 0, sizeof(int), s), "self-test");
@@ -518,7 +524,7 @@ void nwavefunction_compute_density_from_dm(BasisSet *basis, BeckeGrid *grid, dou
 
 // ----------------------------------------------------------- device API
 // rho[p] = sum_{mu,nu} D[mu][nu] phi[mu][p] phi[nu][p]; phi [n][ld] with
-// ld >= padded(npoint) and zero padding, D [n][n] symmetric.
+// ld >= padded(npoint) and zero padding, D [n][n] of any symmetry.
 int napmo_gpu_density(int n, int npoint, const double *phi, long ld, const double *D,
                       double *rho, void *stream) {
   return guarded([&] {

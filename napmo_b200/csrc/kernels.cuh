@@ -48,8 +48,10 @@ struct DensBatchArg {      // density of one molecule
   const double *D;         // [n][n]
   double *rho;             // [npoint]
   const int *keep;         // screening flags or null
-  int n, npoint, vecD, pad;
+  double *fold;            // density_fold_doubles(n): D' of the call
+  int n, npoint;
 };
+size_t density_fold_doubles(int n);  // 0 where the kernel folds D itself
 // Split of an FP64 quadrature into partial sums (quad_plan in quad.cu).
 // n <= 64: class 0 holds nch[0] chunks of chunk[0] points, one warp each.
 // n > 64: the 128 x 128 tiles of the upper triangle in four classes of equal
@@ -90,8 +92,9 @@ struct BatchQueue {
 QuadPlan quad_plan(int n, int npad);
 // Work items of a batched quadrature: a CTA each (n > 64) or 8 chunks (n <= 64).
 int quad_plan_items(int n, const QuadPlan &p);
-cudaError_t launch_density_batch(const DensBatchArg *args, const BatchQueue &q, int grid,
-                                 cudaStream_t s);
+// nfold: the molecules whose D is folded first (0 when none needs it).
+cudaError_t launch_density_batch(const DensBatchArg *args, int nfold, const BatchQueue &q,
+                                 int grid, cudaStream_t s);
 cudaError_t launch_quadrature_batch(const QuadBatchArg *args, const BatchQueue &q, int grid,
                                     cudaStream_t s);
 cudaError_t launch_quadrature_reduce_batch(const QuadBatchArg *args, int nmol, cudaStream_t s);

@@ -27,11 +27,11 @@
 //     2 mt), columns 8 (wc + 4 nt)), so that the fragments left of a diagonal
 //     or ragged tile are spread over the four sub-partitions.
 //
-// density: D is folded onto block-upper-triangular form at 16 x 16 (row tile i
-// takes nu from its own first row on; entries right of its diagonal block
-// count twice, exact for symmetric D); T' = D' phi is folded into the
-// per-point sum with phi[mu][p] as soon as a row tile is complete;
-// deterministic, no atomics.
+// density: D, symmetric or not, is folded onto block-upper-triangular form at
+// 16 x 16 (row tile i takes nu from its own first row on; right of its diagonal
+// block D' = D[mu][nu] + D[nu][mu]); T' = D' phi is folded into the per-point
+// sum with phi[mu][p] as soon as a row tile is complete; deterministic, no
+// atomics.
 // quadrature: split-K over points; chunk partials go to a workspace and a
 // second kernel adds them in a fixed order and writes both triangles, so F is
 // exactly symmetric and bit-reproducible.
@@ -41,12 +41,14 @@
 //
 // Measured (B200, 1965 MHz; before: whole 128 x 128 tiles for every n):
 //   density     H2O (25 functions, 16,500 points)          8.2 ->  4.0 us
-//               C12H26 (310 functions, 1,147,600 points)  6.25 -> 4.62 ms
+//               C12H26 (310 functions, 1,147,600 points)  6.25 -> 4.50 ms
 //   quadrature  H2O, both kernels                           87 ->   11 us
 //               C8H18 (210 functions, 785,200 points)     2.63 -> 1.78 ms
 //               C12H26                                    7.51 -> 5.30 ms
 #include <algorithm>
 #include <cstdint>
+#include <map>
+#include <mutex>
 #include <string>
 
 #include "common.h"
@@ -78,17 +80,12 @@ struct DensSmem {
 constexpr size_t kQuadSmem = sizeof(QuadSmem);
 constexpr size_t kDensSmem = sizeof(DensSmem);
 
-// 16-byte / 8-byte asynchronous global -> shared copies; src_bytes = 0 fills
-// the destination with zeros (rows beyond n) without reading the source.
+// 16-byte asynchronous global -> shared copies; src_bytes = 0 fills the
+// destination with zeros (rows beyond n) without reading the source.
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem),
                "r"(valid ? 16 : 0));
-}
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem, bool valid) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem),
-               "r"(valid ? 8 : 0));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
 template <int N>
@@ -104,8 +101,8 @@ __host__ __device__ constexpr int small_frags(int rt) { return rt * (rt + 1); }
 
 // ------------------------------------------------------------------ density
 // n <= 64: T'[i] = D'[i] phi for 8 points, rho = sum of T' phi.  A warp keeps
-// the fragments of D' (row tile i, k8 step kk >= 2 i; entries right of the
-// diagonal 16 x 16 block doubled) in registers for all its points.
+// the fragments of D' (row tile i, k8 step kk >= 2 i), formed as they are loaded,
+// in registers for all its points.
 template <int RT>
 __device__ __forceinline__ void density_small_frags(int n, const double *__restrict__ D,
                                                     double (&a)[RT * (RT + 1)][4]) {
@@ -118,8 +115,9 @@ __device__ __forceinline__ void density_small_frags(int n, const double *__restr
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int mu = 16 * i + g + 8 * (c & 1), nu = 8 * kk + q + 4 * (c >> 1);
-        const double d = mu < n && nu < n ? __ldg(D + (long)mu * n + nu) : 0.0;
-        a[f][c] = kk >= 2 * i + 2 ? 2.0 * d : d;
+        const bool v = mu < n && nu < n;
+        a[f][c] = v ? __ldg(D + (long)mu * n + nu) : 0.0;
+        if (kk >= 2 * i + 2 && v) a[f][c] += __ldg(D + (long)nu * n + mu);
       }
 }
 
@@ -217,9 +215,9 @@ density_small_kernel(int n, int npoint, const double *__restrict__ phi, long ld,
 // n > 64.  Stages of a CTA: block mb of mu takes nu from mb*BM to n (rounded up
 // to BK = 16), the blocks one after the other; within a block the nu right of
 // the diagonal block come first and the diagonal block's own nu last, in
-// descending order, so that row tile i (16 rows) takes every stage before its
-// own one doubled, its own once, and none after it.  Its phi rows are then in
-// the stage's shared memory, where the fold into rho reads them.
+// descending order, so that row tile i (16 rows) takes every stage up to its
+// own one and none after it.  Its phi rows are then in the stage's shared
+// memory, where the fold into rho reads them.
 struct DensStage {
   int mb, k0;
   int diag;  // the stage's row tile within the diagonal block, or 8 right of it
@@ -249,8 +247,28 @@ __device__ __forceinline__ void density_stage_next(DensStage &s, int nk) {
   }
 }
 
-// rho of the 128 points p0 .. p0 + 127 (one CTA; see density_kernel).
-template <bool kVecD>
+// D' of n > 64, [n][fold_ld(n)]: what density_kernel reads, nu from the first
+// row of mu's 16-row tile on (the rest is left unset), zero in the padding.  A
+// pass of its own, 2.5 us: adding the transposed tile inside density_kernel,
+// whose copies of D it doubles, made that 17 % slower (310 functions).
+__host__ __device__ constexpr int fold_ld(int n) { return (n + 1) / 2 * 2; }
+
+__device__ __forceinline__ void density_fold_body(int n, const double *__restrict__ D,
+                                                  double *__restrict__ out, long e) {
+  const int ldd = fold_ld(n);
+  const int mu = (int)(e / ldd), nu = (int)(e - (long)mu * ldd);
+  if (mu >= n || nu < mu / 16 * 16) return;
+  double d = nu < n ? __ldg(D + (long)mu * n + nu) : 0.0;
+  if (nu < n && nu / 16 > mu / 16) d += __ldg(D + (long)nu * n + mu);
+  out[e] = d;
+}
+
+__global__ void __launch_bounds__(NT)
+density_fold_kernel(int n, const double *__restrict__ D, double *__restrict__ out) {
+  density_fold_body(n, D, out, (long)blockIdx.x * NT + threadIdx.x);
+}
+
+// rho of the 128 points p0 .. p0 + 127 (one CTA; see density_kernel) from D'.
 __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
                                               const double *__restrict__ phi, long ld,
                                               const double *__restrict__ D,
@@ -260,32 +278,21 @@ __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int g = lane >> 2, q = lane & 3;
   const int wr = warp >> 2, wcol = (warp & 3) * 32;
-  const int nblk = (n + BM - 1) / BM;
+  const int nblk = (n + BM - 1) / BM, ldd = fold_ld(n);
   const int nk = (n + BK - 1) / BK;                 // stages of nu over the whole basis
   int nstage = 0;
   for (int mb = 0; mb < nblk; ++mb) nstage += nk - mb * SB;
 
-  // copies of one stage: D' rows (16-byte copies when n is even and D is
-  // 16-byte aligned, else 8-byte; in a diagonal stage only the row tiles that
-  // still take it) and phi rows (16-byte copies; p0 + c is even, ld even)
+  // copies of one stage, 16 bytes each: D' rows (in a diagonal stage only the
+  // row tiles that still take it) and phi rows (p0 + c and ld are even)
   auto load_stage = [&](const DensStage &st, int slot) {
     const int rows = st.diag == SB ? BM : 16 * (st.diag + 1);
-    if (kVecD) {
 #pragma unroll
-      for (int i = 0; i < (BM * BK / 2) / NT; ++i) {
-        const int e = t + NT * i, r = e / (BK / 2), c = (e % (BK / 2)) * 2;
-        const int mu = st.mb * BM + r, nu = st.k0 + c;
-        const bool v = mu < n && nu < n;   // n even: nu + 1 < n as well
-        if (r < rows) cp_async16(&sm.a[slot][r][c], D + (v ? (long)mu * n + nu : 0), v);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < (BM * BK) / NT; ++i) {
-        const int e = t + NT * i, r = e / BK, c = e % BK;
-        const int mu = st.mb * BM + r, nu = st.k0 + c;
-        const bool v = mu < n && nu < n;
-        if (r < rows) cp_async8(&sm.a[slot][r][c], D + (v ? (long)mu * n + nu : 0), v);
-      }
+    for (int i = 0; i < (BM * BK / 2) / NT; ++i) {
+      const int e = t + NT * i, r = e / (BK / 2), c = (e % (BK / 2)) * 2;
+      const int mu = st.mb * BM + r, nu = st.k0 + c;
+      const bool v = mu < n && nu < ldd;
+      if (r < rows) cp_async16(&sm.a[slot][r][c], D + (v ? (long)mu * ldd + nu : 0), v);
     }
 #pragma unroll
     for (int i = 0; i < (BK * BN / 2) / NT; ++i) {
@@ -349,13 +356,6 @@ __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
       if (wr == 1 && mt == 1) next_copies();
       const int i = wr + 2 * mt;                  // row tile within the block
       if (i > st.diag || i >= left) continue;     // warp-uniform
-      if (i == st.diag) {
-        // the part right of the row tile's diagonal block counts twice
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) acc[mt][nt][c] *= 2.0;
-      }
       const int r = 16 * i + g;
 #pragma unroll
       for (int kk = 0; kk < 2; ++kk) {
@@ -405,7 +405,6 @@ __device__ __forceinline__ void density_block(DensSmem &sm, int n, int npoint,
 
 // groups (optional): the 128-point groups to compute (screened plans; the
 // others hold no kept point); keep (optional): rho = 0 at dropped points.
-template <bool kVecD>
 __global__ void __launch_bounds__(NT, 1)
 density_kernel(int n, int npoint, const double *__restrict__ phi, long ld,
                const double *__restrict__ D, double *__restrict__ rho,
@@ -413,7 +412,7 @@ density_kernel(int n, int npoint, const double *__restrict__ phi, long ld,
   extern __shared__ __align__(128) unsigned char smem_raw[];
   DensSmem &sm = *reinterpret_cast<DensSmem *>(smem_raw);
   const int p0 = (groups ? groups[blockIdx.x] : (int)blockIdx.x) * BN;
-  density_block<kVecD>(sm, n, npoint, phi, ld, D, rho, p0, keep);
+  density_block(sm, n, npoint, phi, ld, D, rho, p0, keep);
 }
 
 // --------------------------------------------------------------- quadrature
@@ -865,6 +864,37 @@ QuadPlan quad_plan_slots(int n, int npad, int slots, long *bound = nullptr) {
 // a single tile, four otherwise.
 inline int quad_default_slots(int n) { return n > kSmallN && n <= BM ? 2 * 148 : 4 * 148; }
 
+// Scratch of one call: stream-ordered, so safe with any streams and threads, and
+// a part of the graph when the stream is capturing.  From a pool of the
+// library's own per device, which keeps up to 64 MB between calls (the default
+// pool returns everything to the driver at each synchronisation).
+cudaError_t call_scratch(void **p, size_t bytes, cudaStream_t s) {
+  static std::mutex lock;
+  static std::map<int, cudaMemPool_t> pools;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> hold(lock);
+  cudaMemPool_t &pool = pools[dev];
+  if (!pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    // neither call touches a stream: allowed while some stream is capturing
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    cudaMemPool_t made = nullptr;
+    e = cudaMemPoolCreate(&made, &props);
+    unsigned long long keep = 64ull << 20;
+    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    pool = made;
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+}
+
 inline int pad_points(int npoint) { return ((npoint + BN - 1) / BN) * BN; }
 
 }  // namespace
@@ -884,9 +914,9 @@ cudaError_t launch_density_f64(int n, int npoint, const double *phi, long ld,
     if (blocks == 0) return cudaSuccess;
   }
   if (n <= kSmallN) {
-    // a CTA takes several groups once there are four CTAs per SM
-    const int grid = std::min(blocks, 148 * 4);
-    switch (small_tiles(n)) {
+    // as many CTAs as are resident (registers): each loads D once
+    const int rt = small_tiles(n), grid = std::min(blocks, 148 * (rt == 1 ? 4 : 1));
+    switch (rt) {
       case 1: density_small_kernel<1><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep); break;
       case 2: density_small_kernel<2><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep); break;
       case 3: density_small_kernel<3><<<grid, NT, 0, s>>>(n, npoint, phi, ld, D, rho, groups, blocks, keep); break;
@@ -894,15 +924,22 @@ cudaError_t launch_density_f64(int n, int npoint, const double *phi, long ld,
     }
     return cudaGetLastError();
   }
-  // 16-byte copies of D rows need n even and a 16-byte aligned D
-  const bool vec = n % 2 == 0 && reinterpret_cast<uintptr_t>(D) % 16 == 0;
-  auto kern = vec ? density_kernel<true> : density_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(density_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kDensSmem);
   if (e != cudaSuccess) return e;
-  kern<<<blocks, NT, kDensSmem, s>>>(n, npoint, phi, ld, D, rho, groups, keep);
-  return cudaGetLastError();
+  void *fold = nullptr;
+  const size_t count = density_fold_doubles(n);
+  e = call_scratch(&fold, count * sizeof(double), s);
+  if (e != cudaSuccess) return e;
+  density_fold_kernel<<<(unsigned)((count + NT - 1) / NT), NT, 0, s>>>(n, D, (double *)fold);
+  density_kernel<<<blocks, NT, kDensSmem, s>>>(n, npoint, phi, ld, (const double *)fold, rho,
+                                               groups, keep);
+  e = cudaGetLastError();
+  const cudaError_t ef = cudaFreeAsync(fold, s);
+  return e != cudaSuccess ? e : ef;
 }
+
+size_t density_fold_doubles(int n) { return n > kSmallN ? (size_t)n * fold_ld(n) : 0; }
 
 QuadPlan quad_plan(int n, int npad) { return quad_plan_slots(n, npad, quad_default_slots(n)); }
 
@@ -991,6 +1028,16 @@ __device__ __forceinline__ int cta_pop(const BatchQueue &q, int *slot) {
   return w;
 }
 
+// D' of every molecule (blockIdx.y)
+__global__ void __launch_bounds__(NT)
+density_fold_batch_kernel(const DensBatchArg *__restrict__ args) {
+  const DensBatchArg a = args[blockIdx.y];
+  if (a.n <= kSmallN) return;
+  const long total = (long)a.n * fold_ld(a.n);
+  for (long e = (long)blockIdx.x * NT + threadIdx.x; e < total; e += (long)gridDim.x * NT)
+    density_fold_body(a.n, a.D, a.fold, e);
+}
+
 __global__ void __launch_bounds__(NT, 1)
 density_batch_kernel(const DensBatchArg *__restrict__ args, BatchQueue q) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1006,10 +1053,7 @@ density_batch_kernel(const DensBatchArg *__restrict__ args, BatchQueue q) {
                         a.keep);
       continue;
     }
-    if (a.vecD)
-      density_block<true>(sm, a.n, a.npoint, a.phi, a.ld, a.D, a.rho, it.y * BN, a.keep);
-    else
-      density_block<false>(sm, a.n, a.npoint, a.phi, a.ld, a.D, a.rho, it.y * BN, a.keep);
+    density_block(sm, a.n, a.npoint, a.phi, a.ld, a.fold, a.rho, it.y * BN, a.keep);
   }
 }
 
@@ -1056,9 +1100,10 @@ __global__ void combine_weights_batch_kernel(const WeightBatchArg *__restrict__ 
 
 }  // namespace
 
-cudaError_t launch_density_batch(const DensBatchArg *args, const BatchQueue &q, int grid,
-                                 cudaStream_t s) {
+cudaError_t launch_density_batch(const DensBatchArg *args, int nfold, const BatchQueue &q,
+                                 int grid, cudaStream_t s) {
   if (q.nitems == 0) return cudaSuccess;
+  if (nfold > 0) density_fold_batch_kernel<<<dim3(64, nfold), NT, 0, s>>>(args);
   cudaError_t e = cudaFuncSetAttribute(density_batch_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kDensSmem);

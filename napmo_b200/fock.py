@@ -124,7 +124,7 @@ class FockBuilder(object):
         return x
 
     def density(self, D, stream=None):
-        """rho at every grid point for density matrix D (n x n, symmetric)."""
+        """rho = sum_ij D_ij phi_i phi_j at every grid point (D: n x n)."""
         t = self.torch
         D = self._dev(D, (self.n, self.n))
         rho = t.empty(self.npoint, dtype=t.float64, device='cuda')
