@@ -351,7 +351,9 @@ static int eval_chunk_for(const std::vector<int> &count, const std::vector<Poiss
 // Bucket-sorted (atom, point) pair lists for the evaluation of the potential
 // at the points (x, y, z) (device, all molecules concatenated), into pairs /
 // items; with `keep` only the points whose flag is set.  Built once per grid
-// (and once per screening mask); about 12 bytes per pair.  Synchronises `s`.
+// (and once per screening mask); about 12 bytes per pair.  Synchronises `s`,
+// and the device when the plan has been in use: its buffers are written anew
+// while solves of any stream may still read them.
 int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const double *z,
                      const int *keep, bool nodes, DevBuf<int> &pairs, DevBuf<double2> &pair_u,
                      DevBuf<EvalItem> &items, int &nitems, int &nitems_in, int &chunk,
@@ -362,6 +364,7 @@ int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const 
   for (auto &a : ha) nb += 2 * a.nrad;
   // buffers of an earlier geometry or mask are reused; the pairs' buckets are
   // only needed here and lie in pair_v, which the next evaluation overwrites
+  if (plan->pair_v.p) NAPMO_TRY_CUDA(cudaDeviceSynchronize(), "pair lists");
   NAPMO_TRY_CUDA(plan->pair_v.reserve(d.npair), "pair lists");
   NAPMO_TRY_CUDA(plan->lcut.reserve(nb), "pair lists");
   NAPMO_TRY_CUDA(plan->bucket_count.reserve(nb), "pair lists");
@@ -1344,9 +1347,9 @@ double BeckeGrid_integrate(BeckeGrid *g, double *f) {
 // construction (atomic_grid.cpp:12-51, origin + r u), so the result equals a
 // grid built at the new geometry bit for bit; the device mirror is rewritten
 // in place (no allocation), the Becke weights recomputed and the Poisson
-// plan marked: its next use rebuilds what depends on the positions.  The quadrature weights do not depend
-// on the positions.  No counterpart in nAPMO, which builds a new grid per
-// geometry.  Synchronises the library's host stream.
+// plan marked: its next use rebuilds what depends on the positions.  The
+// quadrature weights do not depend on the positions.  No counterpart in nAPMO,
+// which builds a new grid per geometry.  Synchronises the device.
 int napmo_grid_set_centers(BeckeGrid *g, const double *origin) {
   return guarded([&] {
     NAPMO_REQUIRE(!g->layout.empty() && (int)g->layout.size() == g->ncenter,
@@ -1375,6 +1378,9 @@ int napmo_grid_set_centers(BeckeGrid *g, const double *origin) {
       }
     }
     cudaStream_t s = host_api_stream();
+    // work in flight on any stream reads the points, weights and tables that
+    // are rewritten from here on
+    NAPMO_TRY_CUDA(cudaDeviceSynchronize(), "move grid");
     NAPMO_TRY_CUDA(cudaMemcpyAsync(g->dev.x, x.data(), n * sizeof(double), cudaMemcpyHostToDevice, s),
                    "move grid");
     NAPMO_TRY_CUDA(cudaMemcpyAsync(g->dev.y, y.data(), n * sizeof(double), cudaMemcpyHostToDevice, s),
@@ -1384,11 +1390,7 @@ int napmo_grid_set_centers(BeckeGrid *g, const double *origin) {
     NAPMO_TRY_CUDA(cudaMemcpyAsync(g->dev.origin, g->origin.data(), g->origin.size() * sizeof(double),
                                    cudaMemcpyHostToDevice, s),
                    "move grid");
-    if (g->poisson) {
-      // solves in flight on any stream read the tables that the next use rewrites
-      NAPMO_TRY_CUDA(cudaDeviceSynchronize(), "move grid");
-      g->poisson->moved = true;
-    }
+    if (g->poisson) g->poisson->moved = true;
     ++g->generation;
     return compute_becke(g, s);  // synchronises s before the host vectors go
   });
