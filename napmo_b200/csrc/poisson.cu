@@ -302,7 +302,7 @@ __device__ void spline_dt_col(const double *y, int ys, double *dt, int ds,
 // derivative); Becke-Dickson (op.vsph set): a tabulated on the radial points
 // with its spline derivative (ndpsi.py:58-69).
 __global__ void radial_factor_kernel(PoissonDev P, RadialOp op) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   const int sys = blockIdx.x;
   const PoissonAtom at = P.atoms[P.sys_atom[sys]];
   const int l = P.sys_l[sys];
@@ -497,7 +497,7 @@ __device__ __forceinline__ void ring_wait() {
 template <bool TABLE>
 __global__ void __launch_bounds__(kRadialThreads)
 radial_kernel(PoissonDev P, RadialOp op, const double *__restrict__ ident, int ldi, double *tab) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   const int sys = blockIdx.x;
   const PoissonAtom at = P.atoms[P.sys_atom[sys]];
   const int l = P.sys_l[sys];
@@ -817,7 +817,7 @@ __host__ __device__ constexpr size_t radial_apply_doubles(int n) {
 }
 
 __global__ void __launch_bounds__(kApplyThreads, 2) radial_apply_kernel(PoissonDev P) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   const RadialGroup gr = P.groups[blockIdx.y];
   const int l = gr.l, ncol = 2 * l + 1;
   const int ncols = ncol * gr.natom * P.nbatch;  // natom x nbatch < 2^16, ncol <= 41
@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(kApplyThreads, 2) radial_apply_kernel(PoissonD
 // result with the potential extrapolation (nkinetic.py:48-61,
 // src/grid/radial.cpp:51-192), scaled by `scale` into the evaluation tables.
 __global__ void kinetic_radial_kernel(PoissonDev P, int ncol, double scale) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   const int sys = blockIdx.x;
   const PoissonAtom at = P.atoms[P.sys_atom[sys]];
   const int l = P.sys_l[sys];
@@ -1481,7 +1481,7 @@ constexpr int kRowsThreads = 128;
 __global__ void __launch_bounds__(kRowsThreads) bucket_rows_kernel(PoissonDev P) {
   __shared__ double bound[32];
   __shared__ int s_cut;
-  extern __shared__ double rows[];  // eval_rows(max_lmax) rows; first the terms
+  extern __shared__ __align__(16) double rows[];  // eval_rows(max_lmax) rows; first the terms
   const int bat = blockIdx.y / P.natom;  // solve of a batch
   const PoissonAtom &at = P.atoms[blockIdx.y - bat * P.natom];
   const int b = blockIdx.x, t = threadIdx.x;
@@ -1539,7 +1539,7 @@ template <int LMAX, bool TAILS, bool BATCH>
 __global__ void __launch_bounds__(kEvalChunkMax / (TAILS ? 1 : kEvalPerThread), TAILS ? 1 : 4)
 eval_pairs_kernel(PoissonDev P, const double *__restrict__ gx,
                   const double *__restrict__ gy, const double *__restrict__ gz) {
-  extern __shared__ double cf[];
+  extern __shared__ __align__(16) double cf[];
   constexpr int NP = TAILS ? 1 : kEvalPerThread;
   const EvalItem it = P.items[blockIdx.x + (TAILS ? P.nitems_inner : 0)];
   const PoissonAtom &at = P.atoms[it.atom];
