@@ -35,6 +35,18 @@ cudaStream_t host_api_stream() {
 }
 
 // ------------------------------------------------------------ Poisson plan
+// (atom, point) pairs in class order and their items (build_pair_lists):
+// [0] with node items, [1] by interval, for truncated solves.
+struct PairLists {
+  DevBuf<int> pairs;
+  DevBuf<double2> pair_u;
+  DevBuf<EvalItem> items;
+  int first[2] = {0, 0}, nitems[2] = {0, 0};
+  int nitems_in[2] = {0, 0};   // of them the leading ones are interior
+  int chunk = kEvalChunk;      // pairs per item
+  unsigned long long key = 0;  // screened: serial of the mask's int8 plan (0: none)
+};
+
 struct PoissonPlan {
   PoissonDev d;
   int lmax = -1;
@@ -49,25 +61,13 @@ struct PoissonPlan {
   DevBuf<int> group_atom;
   DevBuf<double> rscr;  // radial-solve scratch of one solve
   DevBuf<double> pg;    // projection scratch of one solve (rho wb w per point)
-  DevBuf<int> pairs;
-  DevBuf<double2> pair_u;  // (u, 1/d) of each interior pair
-  DevBuf<EvalItem> items;
-  int nitems = 0, nitems_in = 0;  // items, of which the first nitems_in are interior
-  int chunk = kEvalChunk;         // pairs per item
+  // of all points, and of those kept by a screening mask (built for the last
+  // mask used; the mask is owned by the caller's int8 plan)
+  PairLists all, screened;
   DevBuf<double> pair_v;
   DevBuf<int> lcut;  // per bucket, for truncated evaluations
-  DevBuf<int> bucket_count;  // pair-list construction
-  bool moved = false;        // the grid's centres moved: centres and pair lists are stale
-  // pair lists of the points kept by a screening mask (built for the last
-  // mask used; the mask is owned by the caller's int8 plan): [0] for truncated
-  // solves, [1] with node buckets for the others
-  struct Screened {
-    DevBuf<int> pairs;
-    DevBuf<double2> pair_u;
-    DevBuf<EvalItem> items;
-    int nitems = 0, nitems_in = 0, chunk = kEvalChunk;
-    unsigned long long key = 0;  // serial of the mask's int8 plan (0: none)
-  } screened[2];
+  DevBuf<int> class_count;  // pair-list construction
+  bool moved = false;       // the grid's centres moved: centres and pair lists are stale
   // Becke-Dickson workspace (source, shell averages, LU factors), kept
   // between calls: an allocation per call would return to the driver at
   // every synchronisation of the caller's loop
@@ -270,7 +270,7 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
     A.mol_npoint = mol_point_off[mol + 1] - mol_point_off[mol];
     plan->max_mol_npoint = std::max(plan->max_mol_npoint, A.mol_npoint);
     A.bucket_off = buckets;
-    buckets += 2 * n;
+    buckets += pair_classes(n);
     A.pair_off = pairs;
     pairs += A.mol_npoint;
     for (int l = 0; l <= lmax; ++l) {
@@ -339,121 +339,120 @@ static int eval_chunk_for(const std::vector<int> &count, const std::vector<Poiss
   long pairs = 0, buckets = 0;
   for (const PoissonAtom &a : ha)
     for (int b = 1; b < a.nrad; ++b) {
-      const int c = count[a.bucket_off + b] + count[a.bucket_off + a.nrad + b];
-      if (c > 0) {
-        pairs += c;
+      const int *c = &count[a.bucket_off + 3 * b];
+      const int total = c[0] + c[1] + c[2];
+      if (total > 0) {
+        pairs += total;
         ++buckets;
       }
     }
-  return buckets > 0 && pairs >= 4096L * buckets ? kEvalChunkMax : kEvalChunk;
+  return buckets > 0 && pairs / buckets >= 4096 ? kEvalChunkMax : kEvalChunk;
 }
 
-// Bucket-sorted (atom, point) pair lists for the evaluation of the potential
-// at the points (x, y, z) (device, all molecules concatenated), into pairs /
-// items; with `keep` only the points whose flag is set.  Built once per grid
-// (and once per screening mask); about 12 bytes per pair.  Synchronises `s`,
-// and the device when the plan has been in use: its buffers are written anew
-// while solves of any stream may still read them.
+// The (atom, point) pairs sorted by the atom's spline intervals, cut into
+// evaluation items; with `keep` only the points whose flag is set.  Two item
+// lists share the pairs: one where an atom's own points are evaluated on their
+// nodes, and one by interval alone for solves that truncate (a truncation's
+// bound holds per interval).  Built once per grid (and once per screening mask);
+// 20 bytes per pair.  Synchronises `s`, and the device when the plan has been in
+// use: its buffers are written anew while solves of any stream may still read
+// them.
 int build_pair_lists(PoissonPlan *plan, const double *x, const double *y, const double *z,
-                     const int *keep, bool nodes, DevBuf<int> &pairs, DevBuf<double2> &pair_u,
-                     DevBuf<EvalItem> &items, int &nitems, int &nitems_in, int &chunk,
-                     cudaStream_t s) {
-  PoissonDev &d = plan->d;
+                     const int *keep, PairLists &l, cudaStream_t s) {
   const std::vector<PoissonAtom> &ha = plan->h_atoms;
-  int nb = 0;
-  for (auto &a : ha) nb += 2 * a.nrad;
-  // buffers of an earlier geometry or mask are reused; the pairs' buckets are
+  int nc = 0;
+  for (auto &a : ha) nc += pair_classes(a.nrad);
+  // buffers of an earlier geometry or mask are reused; the pairs' classes are
   // only needed here and lie in pair_v, which the next evaluation overwrites
   if (plan->pair_v.p) NAPMO_TRY_CUDA(cudaDeviceSynchronize(), "pair lists");
+  PoissonDev d = plan->d;
   NAPMO_TRY_CUDA(plan->pair_v.reserve(d.npair), "pair lists");
-  NAPMO_TRY_CUDA(plan->lcut.reserve(nb), "pair lists");
-  NAPMO_TRY_CUDA(plan->bucket_count.reserve(nb), "pair lists");
-  int *const bucket_of = reinterpret_cast<int *>(plan->pair_v.p);
-  int *const count = plan->bucket_count.p;
-  NAPMO_TRY_CUDA(cudaMemsetAsync(count, 0, nb * sizeof(int), s), "pair lists");
-  NAPMO_TRY_CUDA(launch_pair_buckets(d, plan->max_mol_npoint, x, y, z, keep, nodes, bucket_of,
-                                     count, s),
-                 "pair buckets");
-  std::vector<int> hc(nb);
-  NAPMO_TRY_CUDA(cudaMemcpyAsync(hc.data(), count, nb * sizeof(int), cudaMemcpyDeviceToHost, s),
+  NAPMO_TRY_CUDA(plan->lcut.reserve(nc), "pair lists");
+  NAPMO_TRY_CUDA(plan->class_count.reserve(nc), "pair lists");
+  int *const class_of = reinterpret_cast<int *>(plan->pair_v.p);
+  int *const count = plan->class_count.p;
+  NAPMO_TRY_CUDA(cudaMemsetAsync(count, 0, nc * sizeof(int), s), "pair lists");
+  NAPMO_TRY_CUDA(launch_pair_classes(d, plan->max_mol_npoint, x, y, z, keep, class_of, count, s),
+                 "pair classes");
+  std::vector<int> hc(nc);
+  NAPMO_TRY_CUDA(cudaMemcpyAsync(hc.data(), count, nc * sizeof(int), cudaMemcpyDeviceToHost, s),
                  "pair lists");
   NAPMO_TRY_CUDA(cudaStreamSynchronize(s), "pair lists");
-  // exclusive scan per atom -> bucket starts (relative to the atom's slice)
-  std::vector<int> start(nb);
+  // exclusive scan per atom -> class starts (relative to the atom's slice)
+  std::vector<int> start(nc);
   std::vector<EvalItem> hitems;
-  chunk = eval_chunk_for(hc, ha);
-  for (int a = 0; a < (int)ha.size(); ++a) {
+  l.chunk = eval_chunk_for(hc, ha);
+  for (const PoissonAtom &a : ha) {
     int acc = 0;
-    for (int b = 0; b < 2 * ha[a].nrad; ++b) {
-      const int k = ha[a].bucket_off + b;
+    for (int k = a.bucket_off; k < a.bucket_off + pair_classes(a.nrad); ++k) {
       start[k] = acc;
-      for (int c = 0; c < hc[k]; c += chunk)
-        hitems.push_back(EvalItem{a, b, acc + c, std::min(chunk, hc[k] - c)});
       acc += hc[k];
     }
   }
-  NAPMO_TRY_CUDA(cudaMemcpyAsync(count, start.data(), nb * sizeof(int),  // now the cursor
+  // `classes` classes of atom a from class c on, as items of a bucket
+  auto cut = [&](int a, int bucket, int c, int classes) {
+    const int k = ha[a].bucket_off + c;
+    int total = hc[k];
+    for (int e = 1; e < classes; ++e) total += hc[k + e];
+    for (int e = 0; e < total; e += l.chunk)
+      hitems.push_back(EvalItem{a, bucket, start[k] + e, std::min(l.chunk, total - e)});
+  };
+  const int na = (int)ha.size();
+  hitems.reserve(2 * (d.npair / l.chunk + nc));
+  for (int form = 0; form < 2; ++form) {
+    // interior buckets first, the tails after them: the evaluation runs them as
+    // two kernels, each with the code of its own region only
+    const bool nodes = form == 0;
+    const int lead = nodes ? 1 : 0, classes = nodes ? 1 : 3;
+    l.first[form] = (int)hitems.size();
+    for (int a = 0; a < na; ++a) {
+      const int n = ha[a].nrad;
+      for (int b = 1; b < n; ++b) cut(a, b, 3 * b + lead, classes);
+      if (nodes)
+        for (int j = 0; j < n - 1; ++j) cut(a, n + 1 + j, 3 * j + 2, 2);
+    }
+    l.nitems_in[form] = (int)hitems.size() - l.first[form];
+    for (int a = 0; a < na; ++a)
+      for (int b : {0, ha[a].nrad}) cut(a, b, 3 * b + lead, classes);
+    l.nitems[form] = (int)hitems.size() - l.first[form];
+  }
+  NAPMO_TRY_CUDA(cudaMemcpyAsync(count, start.data(), nc * sizeof(int),  // now the cursor
                                  cudaMemcpyHostToDevice, s),
                  "pair lists");
-  NAPMO_TRY_CUDA(pairs.reserve(d.npair), "pair lists");
-  NAPMO_TRY_CUDA(pair_u.reserve(d.npair), "pair lists");
-  d.pairs = pairs.p;
-  d.pair_u = pair_u.p;
-  NAPMO_TRY_CUDA(launch_pair_scatter(d, plan->max_mol_npoint, x, y, z, bucket_of, count, s),
+  NAPMO_TRY_CUDA(l.pairs.reserve(d.npair), "pair lists");
+  NAPMO_TRY_CUDA(l.pair_u.reserve(d.npair), "pair lists");
+  d.pairs = l.pairs.p;
+  d.pair_u = l.pair_u.p;
+  NAPMO_TRY_CUDA(launch_pair_scatter(d, plan->max_mol_npoint, x, y, z, class_of, count, s),
                  "pair scatter");
-  // interior buckets first, the tails after them: the evaluation runs them as
-  // two kernels, each with the code of its own region only
-  std::stable_partition(hitems.begin(), hitems.end(), [&](const EvalItem &it) {
-    return it.bucket > 0 && it.bucket != ha[it.atom].nrad;
-  });
-  nitems_in = 0;
-  for (const EvalItem &it : hitems) nitems_in += (it.bucket > 0 && it.bucket != ha[it.atom].nrad);
-  NAPMO_TRY_CUDA(items.reserve(hitems.size()), "pair lists");
-  NAPMO_TRY_CUDA(cudaMemcpyAsync(items.p, hitems.data(), hitems.size() * sizeof(EvalItem),
+  NAPMO_TRY_CUDA(l.items.reserve(hitems.size()), "pair lists");
+  NAPMO_TRY_CUDA(cudaMemcpyAsync(l.items.p, hitems.data(), hitems.size() * sizeof(EvalItem),
                                  cudaMemcpyHostToDevice, s),
                  "pair lists");
   NAPMO_TRY_CUDA(cudaStreamSynchronize(s), "pair lists");
-  nitems = (int)hitems.size();
-  d.pair_v = plan->pair_v.p;
+  plan->d.pair_v = plan->pair_v.p;
   return kOk;
 }
 
-// Points the evaluation runs on: all (keep null) or the screened ones, whose
-// lists depend on whether the solves truncate (tol > 0, see pair_bucket).  The
-// two forms agree to rounding and within tol: a capturing stream, where nothing
-// can be built, takes the other if that is what there is.
+// Points and items the evaluation runs on: all points (keep null) or the
+// screened ones, by node or, for truncated solves (tol > 0), by interval.
 static int select_pair_lists(PoissonPlan *p, BeckeGrid *g, const int *keep,
                              unsigned long long key, double tol, cudaStream_t s) {
-  PoissonDev &d = p->d;
-  d.keep = keep;
-  if (!keep) {
-    d.pairs = p->pairs.p;
-    d.pair_u = p->pair_u.p;
-    d.items = p->items.p;
-    d.nitems = p->nitems;
-    d.nitems_inner = p->nitems_in;
-    d.eval_chunk = p->chunk;
-    return kOk;
-  }
-  bool nodes = !(tol > 0.0);
-  if (key != p->screened[nodes].key && key == p->screened[!nodes].key) {
-    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-    NAPMO_TRY_CUDA(cudaStreamIsCapturing(s, &c), "pair lists");
-    if (c != cudaStreamCaptureStatusNone) nodes = !nodes;
-  }
-  PoissonPlan::Screened &l = p->screened[nodes];
-  if (key != l.key) {
+  PairLists &l = keep ? p->screened : p->all;
+  if (keep && key != l.key) {
     l.key = 0;
-    const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, keep, nodes, l.pairs,
-                                    l.pair_u, l.items, l.nitems, l.nitems_in, l.chunk, s);
+    const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, keep, l, s);
     if (st) return st;
     l.key = key;
   }
+  const int form = tol > 0.0;
+  PoissonDev &d = p->d;
+  d.keep = keep;
   d.pairs = l.pairs.p;
   d.pair_u = l.pair_u.p;
-  d.items = l.items.p;
-  d.nitems = l.nitems;
-  d.nitems_inner = l.nitems_in;
+  d.items = l.items.p + l.first[form];
+  d.nitems = l.nitems[form];
+  d.nitems_inner = l.nitems_in[form];
   d.eval_chunk = l.chunk;
   return kOk;
 }
@@ -474,15 +473,9 @@ static int move_poisson_plan(BeckeGrid *g, PoissonPlan *p, cudaStream_t s) {
                                  p->h_atoms.size() * sizeof(PoissonAtom),
                                  cudaMemcpyHostToDevice, s),
                  "move atoms");
-  p->screened[0].key = p->screened[1].key = 0;
-  const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, true, p->pairs, p->pair_u,
-                                  p->items, p->nitems, p->nitems_in, p->chunk, s);
+  p->screened.key = 0;
+  const int st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, p->all, s);
   if (st) return st;
-  d.keep = nullptr;
-  d.items = p->items.p;
-  d.nitems = p->nitems;
-  d.nitems_inner = p->nitems_in;
-  d.eval_chunk = p->chunk;
   p->moved = false;
   return kOk;
 }
@@ -525,16 +518,11 @@ int grid_poisson_plan(BeckeGrid *g, int lmax, cudaStream_t s, PoissonPlan **out)
     delete p;
     return st;
   }
-  st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, true, p->pairs, p->pair_u,
-                        p->items, p->nitems, p->nitems_in, p->chunk, s);
+  st = build_pair_lists(p, g->dev.x, g->dev.y, g->dev.z, nullptr, p->all, s);
   if (st != kOk) {
     delete p;
     return st;
   }
-  p->d.items = p->items.p;
-  p->d.nitems = p->nitems;
-  p->d.nitems_inner = p->nitems_in;
-  p->d.eval_chunk = p->chunk;
   p->lmax = lmax;
   g->poisson = p;
   *out = p;
@@ -597,13 +585,8 @@ int grid_concat(const std::vector<BeckeGrid *> &grids, const std::vector<int> &l
   for (auto &L : g->layout) atoms.push_back(&L);
   int st = build_poisson_plan(atoms, lm, mol_atom_off, o, s, p);
   if (st != kOk) return st;
-  st = build_pair_lists(p, d.x, d.y, d.z, nullptr, true, p->pairs, p->pair_u, p->items, p->nitems,
-                        p->nitems_in, p->chunk, s);
+  st = build_pair_lists(p, d.x, d.y, d.z, nullptr, p->all, s);
   if (st != kOk) return st;
-  p->d.items = p->items.p;
-  p->d.nitems = p->nitems;
-  p->d.nitems_inner = p->nitems_in;
-  p->d.eval_chunk = p->chunk;
   p->lmax = -3;  // not a single-grid cutoff: grid_poisson_plan never reuses it
   NAPMO_TRY_CUDA(cudaStreamSynchronize(s), "batch grid");
   *off = o;

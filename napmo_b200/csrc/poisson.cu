@@ -1135,14 +1135,9 @@ evaluate_kernel(PoissonDev P, int npoint, const double *__restrict__ gx,
 // Bucket of the pair (atom A, point p): 0 below the first radial point, 1 + j
 // inside spline interval j, nrad above the last point -- the same region and
 // interval test as the spline evaluation of the reference
-// (src/horton/cubic_spline.cpp:147-181) -- and nrad + 1 + j for the atom's own
-// points of shell j < nrad - 1, which lie on node j of the spline (not in lists
-// for truncated solves, `nodes` false: those truncate by interval, and rounding
-// puts a node into either of its two).
-__device__ __forceinline__ int pair_bucket(const PoissonAtom &at, int p, double px, double py,
-                                           double pz, bool nodes) {
-  const int own = p - at.point_off;
-  if (nodes && own >= 0 && own < (at.nrad - 1) * at.nang) return at.nrad + 1 + own / at.nang;
+// (src/horton/cubic_spline.cpp:147-181).
+__device__ __forceinline__ int pair_bucket(const PoissonAtom &at, double px, double py,
+                                           double pz) {
   const double dx = px - at.cx, dy = py - at.cy, dz = pz - at.cz;
   const double d = sqrt(dx * dx + dy * dy + dz * dz);
   if (d < at.first_x) return 0;
@@ -1153,26 +1148,42 @@ __device__ __forceinline__ int pair_bucket(const PoissonAtom &at, int p, double 
   return 1 + j;
 }
 
-// Neighbouring points mostly fall in the same bucket of an atom, so the
-// counters are bumped once per group of lanes with equal buckets (the lowest
+// Sort class of the pair, 3 bucket + part.  The atom's own points of shell
+// s < nrad - 1 lie on node s of the spline, and rounding puts each into either
+// of the node's two buckets: part 0 of bucket s + 1 or part 2 of bucket s; part
+// 1 holds everything else.  In class order a node's points are then contiguous,
+// and so is a whole bucket: one order serves both item lists (build_pair_lists).
+__device__ __forceinline__ int pair_class(const PoissonAtom &at, int p, double px, double py,
+                                          double pz) {
+  const int b = pair_bucket(at, px, py, pz), own = p - at.point_off;
+  int part = 1;
+  if (own >= 0 && own < (at.nrad - 1) * at.nang) {
+    const int shell = own / at.nang;
+    if (b == shell + 1) part = 0;
+    if (b == shell) part = 2;
+  }
+  return 3 * b + part;
+}
+
+// Neighbouring points mostly fall in the same class of an atom, so the
+// counters are bumped once per group of lanes with equal classes (the lowest
 // lane adds the group's size): one atomic per group instead of per pair.
 __device__ __forceinline__ int lanes_below(unsigned m) {
   return __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
 }
 
-__global__ void pair_bucket_kernel(PoissonDev P, const double *__restrict__ gx,
-                                   const double *__restrict__ gy,
-                                   const double *__restrict__ gz, const int *__restrict__ keep,
-                                   bool nodes, int *__restrict__ bucket_of,
-                                   int *__restrict__ count) {
+__global__ void pair_class_kernel(PoissonDev P, const double *__restrict__ gx,
+                                  const double *__restrict__ gy,
+                                  const double *__restrict__ gz, const int *__restrict__ keep,
+                                  int *__restrict__ class_of, int *__restrict__ count) {
   const PoissonAtom &at = P.atoms[blockIdx.y];
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = q < at.mol_npoint;
   int b = -1;
   if (in) {
     const int p = at.mol_point_start + q;
-    if (!keep || keep[p]) b = pair_bucket(at, p, gx[p], gy[p], gz[p], nodes);  // -1: screened out
-    bucket_of[at.pair_off + q] = b;
+    if (!keep || keep[p]) b = pair_class(at, p, gx[p], gy[p], gz[p]);  // -1: screened out
+    class_of[at.pair_off + q] = b;
   }
   const unsigned group = __match_any_sync(0xffffffffu, b);
   if (b >= 0 && lanes_below(group) == 0) atomicAdd(&count[at.bucket_off + b], __popc(group));
@@ -1188,24 +1199,27 @@ __device__ __forceinline__ double pair_distance(const PoissonAtom &at, const dou
 __global__ void pair_scatter_kernel(PoissonDev P, const double *__restrict__ gx,
                                     const double *__restrict__ gy,
                                     const double *__restrict__ gz,
-                                    const int *__restrict__ bucket_of,
+                                    const int *__restrict__ class_of,
                                     int *__restrict__ cursor) {
   const PoissonAtom &at = P.atoms[blockIdx.y];
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = q < at.mol_npoint ? bucket_of[at.pair_off + q] : -1;
-  const unsigned group = __match_any_sync(0xffffffffu, b);
+  const int c = q < at.mol_npoint ? class_of[at.pair_off + q] : -1;
+  const unsigned group = __match_any_sync(0xffffffffu, c);
   const int leader = __ffs(group) - 1;
   int base = 0;
-  if (b >= 0 && (int)(threadIdx.x & 31) == leader)
-    base = atomicAdd(&cursor[at.bucket_off + b], __popc(group));
+  if (c >= 0 && (int)(threadIdx.x & 31) == leader)
+    base = atomicAdd(&cursor[at.bucket_off + c], __popc(group));
   base = __shfl_sync(0xffffffffu, base, leader);
-  if (b >= 0) {
+  if (c >= 0) {
     const long slot = at.pair_off + base + lanes_below(group);
     const int p = at.mol_point_start + q;
     P.pairs[slot] = p;
-    if (b > 0 && b != at.nrad) {  // interior: the evaluation's u and 1/d
+    // what the evaluation of an interval (u, 1/d) or a node (1/d) reads
+    const int b = c / 3;
+    const bool inside = b > 0 && b < at.nrad;
+    if (inside || c - 3 * b == 2) {
       const double d = pair_distance(at, gx, gy, gz, p);
-      P.pair_u[slot] = make_double2(b < at.nrad ? rt_inv(at.rt, d) - (b - 1) : 0.0, 1.0 / d);
+      P.pair_u[slot] = make_double2(inside ? rt_inv(at.rt, d) - (b - 1) : 0.0, 1.0 / d);
     }
   }
 }
@@ -1887,19 +1901,19 @@ cudaError_t launch_shell_average(const PoissonDev &P, const double *f, const dou
   return cudaGetLastError();
 }
 
-cudaError_t launch_pair_buckets(const PoissonDev &P, int max_mol_npoint, const double *x,
-                                const double *y, const double *z, const int *keep, bool nodes,
-                                int *bucket_of, int *count, cudaStream_t s) {
+cudaError_t launch_pair_classes(const PoissonDev &P, int max_mol_npoint, const double *x,
+                                const double *y, const double *z, const int *keep,
+                                int *class_of, int *count, cudaStream_t s) {
   dim3 grid((max_mol_npoint + 255) / 256, P.natom);
-  pair_bucket_kernel<<<grid, 256, 0, s>>>(P, x, y, z, keep, nodes, bucket_of, count);
+  pair_class_kernel<<<grid, 256, 0, s>>>(P, x, y, z, keep, class_of, count);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pair_scatter(const PoissonDev &P, int max_mol_npoint, const double *x,
-                                const double *y, const double *z, const int *bucket_of,
+                                const double *y, const double *z, const int *class_of,
                                 int *cursor, cudaStream_t s) {
   dim3 grid((max_mol_npoint + 255) / 256, P.natom);
-  pair_scatter_kernel<<<grid, 256, 0, s>>>(P, x, y, z, bucket_of, cursor);
+  pair_scatter_kernel<<<grid, 256, 0, s>>>(P, x, y, z, class_of, cursor);
   return cudaGetLastError();
 }
 

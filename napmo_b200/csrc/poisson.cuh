@@ -24,8 +24,8 @@ struct PoissonAtom {
   int amp_off;    // [lsize][2] left / right extrapolation amplitudes (scaled)
   int raw_off;    // [lsize][nrad] solution values y and t-derivatives dt
   int mol_point_start, mol_npoint;  // points of this atom's molecule
-  int bucket_off;  // [2 nrad] buckets: 0 left tail, 1 + j interval j, nrad right tail,
-                   // nrad + 1 + j own points on node j < nrad - 1
+  int bucket_off;  // buckets: 0 left tail, 1 + j interval j, nrad right tail; room for
+                   // pair_classes(nrad)
   int sys_off;     // radial system of (this atom, l) = sys_off + l
   long pair_off;   // this atom's slice of the (atom, point) pair arrays
   long gop_off;    // radial operators of this radial grid: [lmax + 1][rows][ld]
@@ -33,8 +33,12 @@ struct PoissonAtom {
   long scr_off;    // radial-solve scratch: [3 nrad][lsize]
 };
 
+// Sort classes of an atom's pairs: three parts per bucket (pair_class).
+__host__ __device__ constexpr int pair_classes(int nrad) { return 3 * (nrad + 1); }
+
 // One CTA of the bucketed evaluation: `count` (<= the plan's chunk) pairs of one
-// atom that share one spline interval (or tail) of that atom.
+// atom that share one spline interval (or tail) of that atom, or (bucket nrad +
+// 1 + j) its own points on node j.
 struct EvalItem {
   int atom, bucket, start, count;
 };
@@ -114,8 +118,8 @@ struct PoissonDev {
   int nitems = 0;
   int nitems_inner = 0;        // items [0, nitems_inner) lie inside their atom's grid
   int eval_chunk = kEvalChunk;  // pairs per item (<= kEvalChunkMax); CTA = chunk / 4 threads
-  int *pairs = nullptr;        // point index, bucket-sorted per atom
-  double2 *pair_u = nullptr;   // (u, 1/d) of each interior pair (slot order)
+  int *pairs = nullptr;        // point index, in class order per atom
+  double2 *pair_u = nullptr;   // (u, 1/d) of each interior or node pair (slot order)
   EvalItem *items = nullptr;
   double *pair_v = nullptr;    // [atom][molecule point] contribution
   // Truncation of the bucketed evaluation: with lcut null every (l, m) <=
@@ -183,19 +187,18 @@ cudaError_t launch_kinetic_radial(const PoissonDev &P, double scale, cudaStream_
 // directions (AtomicGrid.spherical_average of f wb); out at rad_off / kRadSlots.
 cudaError_t launch_shell_average(const PoissonDev &P, const double *f, const double *wb,
                                  const double *w, double *out, cudaStream_t s);
-// Pair-list construction: bucket of every (atom, point) pair and the bucket
-// populations (count[atom.bucket_off + b], atomics on integers), then the
-// bucket-sorted point lists (order inside a bucket is irrelevant: each pair
+// Pair-list construction: class of every (atom, point) pair and the class
+// populations (count[atom.bucket_off + c], atomics on integers), then the
+// class-sorted point lists (order inside a class is irrelevant: each pair
 // writes its own slot of pair_v).
-// With keep non-null, points whose flag is 0 get no pair (bucket -1).
-cudaError_t launch_pair_buckets(const PoissonDev &P, int max_mol_npoint, const double *x,
-                                const double *y, const double *z, const int *keep, bool nodes,
-                                int *bucket_of, int *count, cudaStream_t s);
-// The scatter also stores, for the pairs of interior buckets, the spline
-// interval coordinate u = rt_inv(|p - A|) - j and 1 / |p - A| in P.pair_u
-// (slot order).
+// With keep non-null, points whose flag is 0 get no pair (class -1).
+cudaError_t launch_pair_classes(const PoissonDev &P, int max_mol_npoint, const double *x,
+                                const double *y, const double *z, const int *keep,
+                                int *class_of, int *count, cudaStream_t s);
+// The scatter also stores, for interior and node pairs, the spline interval
+// coordinate u = rt_inv(|p - A|) - j and 1 / |p - A| in P.pair_u (slot order).
 cudaError_t launch_pair_scatter(const PoissonDev &P, int max_mol_npoint, const double *x,
-                                const double *y, const double *z, const int *bucket_of,
+                                const double *y, const double *z, const int *class_of,
                                 int *cursor, cudaStream_t s);
 // spline tables -> potential at every grid point (out = or += ).  Uses the
 // bucketed pair lists when P.items is set, the point-parallel kernel otherwise.
