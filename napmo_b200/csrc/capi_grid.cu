@@ -98,17 +98,15 @@ static void ytable(const std::vector<double> &ang, int nang, int lmax,
   }
 }
 
-// The radial operators of a plan whose atoms (h_atoms, d.atoms) and radial tables
-// are set: one set per distinct radial grid, whatever its atoms.  *use = false,
-// with nothing built, for grids beyond kRadialOpMax points or operators beyond
-// kRadialOpBytes in all: those plans substitute per solve.
-constexpr size_t kRadialOpBytes = 512ull << 20;
+// The radial operators of the plan's atoms of up to kRadialOpMax radial points,
+// whose radial tables are set: one set per distinct radial grid, so that what an
+// atom's solve does depends on its own grid alone.  *built = false, with nothing
+// kept, when the device has no room for them.
 static int build_radial_operators(PoissonPlan *plan, const std::vector<double> &rad,
-                                  cudaStream_t s, bool *use) {
+                                  cudaStream_t s, bool *built) {
   PoissonDev &d = plan->d;
   std::vector<PoissonAtom> &ha = plan->h_atoms;
-  *use = false;
-  if (d.natom == 0 || d.max_nrad > kRadialOpMax) return kOk;
+  *built = true;
   // atoms by radial grid (radius, weight and the three derivatives: the first
   // five tables), then by lmax
   auto less = [&](int a, int b) {
@@ -118,11 +116,12 @@ static int build_radial_operators(PoissonPlan *plan, const std::vector<double> &
     return c != 0 ? c < 0 : false;
   };
   std::map<int, std::map<int, std::vector<int>>, decltype(less)> kinds(less);
-  for (int a = 0; a < d.natom; ++a) kinds[a][ha[a].lmax].push_back(a);
+  for (int a = 0; a < d.natom; ++a)
+    if (ha[a].nrad <= kRadialOpMax) kinds[a][ha[a].lmax].push_back(a);
+  if (kinds.empty()) return kOk;
   std::vector<RadialGroup> groups;
   std::vector<int> order, sys_atom, sys_l;
   size_t total = 0;
-  d.max_group_cols = 0;
   for (auto &kind : kinds) {
     const int n = ha[kind.first].nrad;
     int top = 0;  // an atom with the kind's largest lmax
@@ -137,27 +136,38 @@ static int build_radial_operators(PoissonPlan *plan, const std::vector<double> &
       top = by.second[0];
       d.max_group_cols = std::max(d.max_group_cols, count * (2 * lmax + 1));
     }
+    d.max_op_nrad = std::max(d.max_op_nrad, n);
     for (int l = 0; l <= ha[top].lmax; ++l) {
       sys_atom.push_back(top);
       sys_l.push_back(l);
     }
     total += (size_t)(ha[top].lmax + 1) * radial_op_rows(n) * radial_op_ld(n);
   }
-  if (total * sizeof(double) > kRadialOpBytes || groups.size() > 65535) return kOk;
-  // one temporary: the kinds' systems, their LU factors and the table's scratch
-  const int nk = (int)sys_atom.size();
-  const size_t rows = (size_t)nk * d.lu_stride;
-  const size_t doubles = rows * (kW + kKL) + radial_op_tmp_doubles(nk, d.max_nrad);
+  // the kinds' systems in slices, of which one temporary holds the LU factors
+  // and the table's scratch (at most 256 MB)
+  const int nk = (int)sys_atom.size(), stride = 2 * d.max_op_nrad;
+  const size_t per = (size_t)stride * (kW + kKL) + (size_t)d.max_op_nrad * d.max_op_nrad;
+  const int slice = std::min<size_t>(nk, std::max<size_t>((32ull << 20) / per, 1));
+  const size_t lu = (size_t)slice * stride;
   DevBuf<double> tmp;
   DevBuf<int> itmp;
+  // (the temporaries first: after the operators they took a fresh 2 MB block of
+  // the driver, and freeing that cost an H2O 50 x 110 plan 0.7 of 2.6 ms)
+  cudaError_t e = tmp.alloc(lu * (kW + kKL) + radial_op_tmp_doubles(slice, d.max_op_nrad));
+  if (e == cudaSuccess) e = itmp.alloc(2 * (size_t)nk + lu);
+  if (e == cudaSuccess) e = plan->gop.alloc(total);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    plan->gop.reset();
+    *built = false;
+    return kOk;
+  }
+  NAPMO_TRY_CUDA(e, "alloc radial operators");
   std::vector<int> sys(sys_atom);
   sys.insert(sys.end(), sys_l.begin(), sys_l.end());
-  NAPMO_TRY_CUDA(tmp.alloc(doubles), "alloc radial operators");
-  NAPMO_TRY_CUDA(itmp.alloc(2 * (size_t)nk + rows), "alloc radial operators");
   NAPMO_TRY_CUDA(cudaMemcpyAsync(itmp.p, sys.data(), sys.size() * sizeof(int),
                                  cudaMemcpyHostToDevice, s),
                  "upload");
-  NAPMO_TRY_CUDA(plan->gop.alloc(total), "alloc radial operators");
   NAPMO_TRY_CUDA(cudaMemsetAsync(plan->gop.p, 0, total * sizeof(double), s), "radial operators");
   NAPMO_TRY_CUDA(plan->groups.upload(groups, s), "upload");
   NAPMO_TRY_CUDA(plan->group_atom.upload(order, s), "upload");
@@ -166,20 +176,23 @@ static int build_radial_operators(PoissonPlan *plan, const std::vector<double> &
                  "upload atoms");
   PoissonDev k = d;
   k.gop = plan->gop.p;
-  k.nsys = nk;
-  k.sys_atom = itmp.p;
-  k.sys_l = itmp.p + nk;
+  k.max_nrad = d.max_op_nrad;
+  k.lu_stride = stride;
   k.lpiv = itmp.p + 2 * nk;
   k.lu = tmp.p;
-  k.lmul = k.lu + rows * kW;
-  NAPMO_TRY_CUDA(launch_poisson_factor(k, s), "radial LU");
-  NAPMO_TRY_CUDA(launch_radial_operators(k, k.lmul + rows * kKL, s), "radial operators");
+  k.lmul = k.lu + lu * kW;
+  for (int s0 = 0; s0 < nk; s0 += slice) {
+    k.nsys = std::min(slice, nk - s0);
+    k.sys_atom = itmp.p + s0;
+    k.sys_l = itmp.p + nk + s0;
+    NAPMO_TRY_CUDA(launch_poisson_factor(k, s), "radial LU");
+    NAPMO_TRY_CUDA(launch_radial_operators(k, k.lmul + lu * kKL, s), "radial operators");
+  }
   NAPMO_TRY_CUDA(cudaStreamSynchronize(s), "radial operators");
   d.gop = plan->gop.p;
   d.groups = plan->groups.p;
   d.group_atom = plan->group_atom.p;
   d.ngroup = (int)groups.size();
-  *use = true;
   return kOk;
 }
 
@@ -264,7 +277,6 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
     A.scr_off = scr;
     scr += 3L * n * lsize;
     npts = std::max(npts, (long)L.point_off + (long)n * L.nang);
-    A.sys_off = (int)sys_atom.size();
     const int mol = atom_mol[a];
     A.mol_point_start = mol_point_off[mol];
     A.mol_npoint = mol_point_off[mol + 1] - mol_point_off[mol];
@@ -273,13 +285,19 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
     buckets += pair_classes(n);
     A.pair_off = pairs;
     pairs += A.mol_npoint;
-    for (int l = 0; l <= lmax; ++l) {
-      sys_atom.push_back(a);
-      sys_l.push_back(l);
-    }
     d.max_lmax = std::max(d.max_lmax, lmax);
     d.max_nrad = std::max(d.max_nrad, n);
     d.max_nang = std::max(d.max_nang, L.nang);
+  }
+  // the systems that are solved by substitution come first
+  for (bool sub : {true, false}) {
+    for (int a = 0; a < natom; ++a)
+      if ((ha[a].nrad > kRadialOpMax) == sub)
+        for (int l = 0; l <= ha[a].lmax; ++l) {
+          sys_atom.push_back(a);
+          sys_l.push_back(l);
+        }
+    if (sub) d.nsub = (int)sys_atom.size();
   }
   d.nsys = (int)sys_atom.size();
   NAPMO_TRY_CUDA(plan->atoms.upload(ha, s), "upload atoms");
@@ -314,17 +332,21 @@ int build_poisson_plan(const std::vector<const AtomLayout *> &atoms,
   d.pg = plan->pg.p;
   d.npair = pairs;
   d.lu_stride = 2 * d.max_nrad;
-  bool use = false;
-  int st = build_radial_operators(plan, rad, s, &use);
-  if (st != kOk || use) return st;
-  // LU factors of the radial systems (they depend on the grid only)
-  NAPMO_TRY_CUDA(plan->lu.alloc((size_t)d.nsys * d.lu_stride * kW), "alloc radial LU");
-  NAPMO_TRY_CUDA(plan->lmul.alloc((size_t)d.nsys * d.lu_stride * kKL), "alloc radial LU");
-  NAPMO_TRY_CUDA(plan->lpiv.alloc((size_t)d.nsys * d.lu_stride), "alloc radial LU");
+  bool built = false;
+  const int st = build_radial_operators(plan, rad, s, &built);
+  if (st != kOk) return st;
+  if (!built) d.nsub = d.nsys;
+  if (d.nsub == 0) return kOk;
+  // LU factors of the substituted systems (they depend on the grid only)
+  NAPMO_TRY_CUDA(plan->lu.alloc((size_t)d.nsub * d.lu_stride * kW), "alloc radial LU");
+  NAPMO_TRY_CUDA(plan->lmul.alloc((size_t)d.nsub * d.lu_stride * kKL), "alloc radial LU");
+  NAPMO_TRY_CUDA(plan->lpiv.alloc((size_t)d.nsub * d.lu_stride), "alloc radial LU");
   d.lu = plan->lu.p;
   d.lmul = plan->lmul.p;
   d.lpiv = plan->lpiv.p;
-  NAPMO_TRY_CUDA(launch_poisson_factor(d, s), "radial LU");
+  PoissonDev sub = d;
+  sub.nsys = d.nsub;
+  NAPMO_TRY_CUDA(launch_poisson_factor(sub, s), "radial LU");
   return kOk;
 }
 
@@ -682,7 +704,7 @@ int run_poisson_many(BeckeGrid *g, PoissonPlan *p, int k, const double *rho_dev,
   int st = select_pair_lists(p, g, keep, key, tol, s);
   if (st) return st;
   const PoissonDev &d = p->d;
-  const size_t nscr = d.gop ? 0 : p->rscr.n;  // the operators need no scratch
+  const size_t nscr = d.nsub ? p->rscr.n : 0;  // the operators need no scratch
   const size_t nd = p->proj.n + p->spl.n + p->rows.n + p->amp.n + p->pair_v.n + nscr +
                     p->pg.n;
   const size_t per = nd * sizeof(double) + p->lcut.n * sizeof(int);

@@ -13,8 +13,8 @@
 //    (l, m) with scipy's sparse LU), so their composition is tabulated once per
 //    radial grid and l by solving for unit f (radial_kernel<true>), and a solve
 //    is one FP64 tensor product per (radial grid, l) (radial_apply_kernel).
-//    Radial grids beyond kRadialOpMax points and the Becke-Dickson correction,
-//    whose matrix changes with every call, substitute per solve
+//    Atoms of more than kRadialOpMax radial points and the Becke-Dickson
+//    correction, whose matrix changes with every call, substitute per solve
 //    (radial_kernel<false>).  The solution splines are written as scaled cubic
 //    coefficients for step 3 and as raw (y, dy/dt) for the Python API.
 // 3. evaluate: v(p) = sum_A sum_lm s_lm(|p - A|) sqrt(2l+1)/sqrt(4 pi)
@@ -1867,16 +1867,26 @@ cudaError_t launch_radial_operators(const PoissonDev &P, double *tmp, cudaStream
 }
 
 cudaError_t launch_poisson_radial(const PoissonDev &P, cudaStream_t s) {
-  if (!P.gop) return launch_radial_solve(P, RadialOp(), s);
+  if (P.nsub > 0) {
+    PoissonDev sub = P;
+    sub.nsys = P.nsub;
+    const cudaError_t e = launch_radial_solve(sub, RadialOp(), s);
+    if (e != cudaSuccess) return e;
+  }
   if (P.ngroup == 0) return cudaSuccess;
   const long tiles = ((long)P.max_group_cols * P.nbatch + kApplyCols - 1) / kApplyCols;
-  const size_t smem = radial_apply_doubles(P.max_nrad) * sizeof(double);
-  if (tiles > 0x7fffffffL || P.ngroup > 65535 || smem > kMaxSmem) return cudaErrorInvalidValue;
+  const size_t smem = radial_apply_doubles(P.max_op_nrad) * sizeof(double);
+  if (tiles > 0x7fffffffL || smem > kMaxSmem) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(radial_apply_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  radial_apply_kernel<<<dim3((unsigned)tiles, P.ngroup), kApplyThreads, smem, s>>>(P);
-  return cudaGetLastError();
+  for (int g0 = 0; g0 < P.ngroup && e == cudaSuccess; g0 += 65535) {
+    PoissonDev part = P;
+    part.groups = P.groups + g0;
+    radial_apply_kernel<<<dim3((unsigned)tiles, std::min(P.ngroup - g0, 65535)), kApplyThreads,
+                          smem, s>>>(part);
+    e = cudaGetLastError();
+  }
+  return e;
 }
 
 cudaError_t launch_kinetic_radial(const PoissonDev &P, double scale, cudaStream_t s) {

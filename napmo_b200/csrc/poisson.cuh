@@ -26,7 +26,6 @@ struct PoissonAtom {
   int mol_point_start, mol_npoint;  // points of this atom's molecule
   int bucket_off;  // buckets: 0 left tail, 1 + j interval j, nrad right tail; room for
                    // pair_classes(nrad)
-  int sys_off;     // radial system of (this atom, l) = sys_off + l
   long pair_off;   // this atom's slice of the (atom, point) pair arrays
   long gop_off;    // radial operators of this radial grid: [lmax + 1][rows][ld]
   long rows_off;   // evaluation rows: [nrad - 1][eval_rows_doubles(lmax)]
@@ -76,7 +75,8 @@ __host__ __device__ constexpr int radial_op_rows(int n) { return (2 * n + 15) / 
 __host__ __device__ constexpr int radial_op_ld(int n) { return (n + 7) / 8 * 8; }
 
 struct PoissonDev {
-  int natom = 0, nmol = 0, nsys = 0;
+  int natom = 0, nmol = 0;
+  int nsys = 0, nsub = 0;        // radial systems; the first nsub are solved by substitution
   int max_lmax = 0, max_nrad = 0, max_nang = 0;
   PoissonAtom *atoms = nullptr;
   int *mol_atom_off = nullptr;   // nmol + 1
@@ -91,13 +91,14 @@ struct PoissonDev {
   double *amp = nullptr;
   double *raw_y = nullptr;
   double *raw_dt = nullptr;
-  // Radial operators, one set per distinct radial grid (null: the Poisson
-  // solves substitute with the LU factors below instead)
+  // Radial operators, one set per distinct radial grid of at most kRadialOpMax
+  // points, for the systems from nsub on
   double *gop = nullptr;
   RadialGroup *groups = nullptr;
   int *group_atom = nullptr;
-  int ngroup = 0, max_group_cols = 0;  // largest natom (2 l + 1)
-  // LU factors of the radial FEM systems (built once per grid): per system
+  int ngroup = 0, max_op_nrad = 0;
+  int max_group_cols = 0;  // largest natom (2 l + 1)
+  // LU factors of the substituted FEM systems (built once per grid): per system
   // the band [2 nrad][kW], multipliers [2 nrad][3], pivots [2 nrad]; strides
   // use lu_stride = 2 max_nrad rows
   double *lu = nullptr;
