@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "device_types.h"
+#include "quad_plan.h"
 
 namespace napmo {
 
@@ -52,15 +53,6 @@ struct DensBatchArg {      // density of one molecule
   int n, npoint;
 };
 size_t density_fold_doubles(int n);  // 0 where the kernel folds D itself
-// Split of an FP64 quadrature into partial sums (quad_plan in quad.cu).
-// n <= 64: class 0 holds nch[0] chunks of chunk[0] points, one warp each.
-// n > 64: the 128 x 128 tiles of the upper triangle in four classes of equal
-// cost (right of the diagonal: full, last column; diagonal: full, last); class
-// c has ntile[c] tiles, each split into nch[c] chunks of chunk[c] points, its
-// CTAs numbered from first[c], tile fastest; CTA b writes workspace slot b.
-struct QuadPlan {
-  int ntile[4], nch[4], chunk[4], first[5];
-};
 struct QuadBatchArg {      // quadrature of one molecule
   const double *phi;       // [n][ld]
   long ld;

@@ -54,13 +54,14 @@
 #include "common.h"
 #include "dmma.cuh"
 #include "kernels.cuh"
+#include "quad_plan.h"
 
 namespace napmo {
 
 namespace {
 
-constexpr int BM = 128, BN = 128, NT = 256;
-constexpr int BK = 16;                 // points (quadrature) / functions (density) per stage
+constexpr int BM = kQuadTile, BN = kQuadTile, NT = 256;
+constexpr int BK = kQuadStage;         // points (quadrature) / functions (density) per stage
 constexpr int NS = 4;                  // stages of the cp.async ring
 constexpr int LDA = BK + 4;            // [row][k] tiles: stride 20 doubles
 constexpr int LDB = BN + 4;            // density phi tile [nu][p]: stride 132 doubles
@@ -93,11 +94,7 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-constexpr int kSmallN = 64;            // whole triangle of fragments per warp up to this n
 constexpr int kWarps = NT / 32;
-// row tiles of 16 that cover n <= kSmallN, and their upper-triangle fragments
-__host__ __device__ constexpr int small_tiles(int n) { return (n + 15) / 16; }
-__host__ __device__ constexpr int small_frags(int rt) { return rt * (rt + 1); }
 
 // ------------------------------------------------------------------ density
 // n <= 64: T'[i] = D'[i] phi for 8 points, rho = sum of T' phi.  A warp keeps
@@ -496,20 +493,6 @@ quadrature_small_kernel(int n, int npoint_pad, const double *__restrict__ phi,
     quadrature_small_chunk<RT, false>(n, npoint_pad, phi, phib, ld, wv, chunk, work, blocks, ck);
 }
 
-// n > 64.  Tile `t` of class `c` (QuadPlan) of nblk x nblk blocks.
-__device__ __forceinline__ void quad_tile(int c, int t, int nblk, int &mb, int &nb) {
-  if (c == 0) {
-    nb = 1;
-    while (t >= nb) t -= nb++;
-    mb = t;
-  } else if (c == 1) {
-    mb = t;
-    nb = nblk - 1;
-  } else {
-    mb = nb = c == 2 ? t : nblk - 1;
-  }
-}
-
 // Fragments of one warp in a diagonal tile of R row tiles (16 rows) and C = 2 R
 // or 2 R - 1 column tiles (8 columns).  Row tile i has the C - 2 i fragments
 // from column 2 i on; row tiles p and R - 1 - p together have twice L = C - R
@@ -798,72 +781,6 @@ __global__ void combine_weights_kernel(int npoint, const double *__restrict__ wb
   wv[p] = wb[p] * w[p] * pot;
 }
 
-// Cost of a stage of one tile: DMMA instructions per k8 step of the busiest
-// sub-partition (warps w and w + 4), plus the stage's fixed part (barrier and
-// copies, about 4 of them).
-inline int quad_tile_cost(int n, int nblk, int cls) {
-  const bool ragged = cls == 1 || cls == 3;
-  const int cols = ragged ? n - (nblk - 1) * BN : BN;
-  const int C = (cols + 7) / 8, R = (cols + 15) / 16;
-  const int groups4 = (C + 3) / 4 * 4, frags3 = (C - R + 1 + 2) / 3 * 3;
-  return 4 + (cls < 2 ? 2 * groups4 : (R > 4 ? 2 : 1) * frags3);
-}
-
-// The split for at most `slots` partial tiles (n > 64) or chunks (n <= 64).
-// *bound (optional) receives the most slots that any range of at most npad
-// points uses: a shorter range can be cut into more chunks (chunk lengths are
-// rounded up to 16 points), up to one per 16 points and the counts below.
-QuadPlan quad_plan_slots(int n, int npad, int slots, long *bound = nullptr) {
-  QuadPlan p = {};
-  if (bound) *bound = 0;
-  auto split = [&](int c) {  // chunk length and count for at most nch[c] chunks
-    if (bound) *bound += (long)p.ntile[c] * std::max(std::min(p.nch[c], npad / BK), 1);
-    int chunk = (npad + p.nch[c] - 1) / p.nch[c];
-    chunk = std::max((chunk + BK - 1) / BK * BK, BK);
-    p.chunk[c] = chunk;
-    p.nch[c] = (npad + chunk - 1) / chunk;
-  };
-  if (n <= kSmallN) {
-    p.ntile[0] = 1;
-    p.nch[0] = slots;
-    split(0);
-    for (int c = 1; c < 5; ++c) p.first[c] = p.nch[0];
-    return p;
-  }
-  const int nblk = (n + BM - 1) / BM;
-  p.ntile[0] = (nblk - 1) * (nblk - 2) / 2;
-  p.ntile[1] = nblk - 1;
-  p.ntile[2] = nblk - 1;
-  p.ntile[3] = 1;
-  long total = 0;
-  int cost[4];
-  for (int c = 0; c < 4; ++c) {
-    cost[c] = quad_tile_cost(n, nblk, c);
-    total += (long)cost[c] * p.ntile[c];
-  }
-  // chunks in proportion to the cost, so that all CTAs take about as long
-  for (int s = slots;; --s) {
-    long used = 0;
-    bool single = true;
-    for (int c = 0; c < 4; ++c) {
-      p.nch[c] = (int)std::max<long>((long)s * cost[c] / total, 1);
-      used += (long)p.nch[c] * p.ntile[c];
-      single = single && p.nch[c] == 1;
-    }
-    if (used <= slots || single) break;
-  }
-  for (int c = 0; c < 4; ++c) {
-    split(c);
-    p.first[c + 1] = p.first[c] + p.nch[c] * p.ntile[c];
-  }
-  return p;
-}
-
-// Slots: n <= 64 (a warp per chunk) four warps per SM; n > 64 (a CTA per slot,
-// one CTA per SM at these register counts) two full waves over the 148 SMs for
-// a single tile, four otherwise.
-inline int quad_default_slots(int n) { return n > kSmallN && n <= BM ? 2 * 148 : 4 * 148; }
-
 // Scratch of one call: stream-ordered, so safe with any streams and threads, and
 // a part of the graph when the stream is capturing.  From a pool of the
 // library's own per device, which keeps up to 64 MB between calls (the default
@@ -973,9 +890,7 @@ cudaError_t quadrature_launch(const QuadPlan &plan, int n, int npad, const doubl
 }
 
 size_t quadrature_workspace_bytes(int n, int npoint) {
-  long slots = 0;
-  quad_plan_slots(n, pad_points(npoint), quad_default_slots(n), &slots);
-  return slots * (n <= kSmallN ? 128 * small_frags(small_tiles(n)) : BM * BN) * sizeof(double);
+  return quad_workspace_doubles(n, pad_points(npoint)) * sizeof(double);
 }
 
 cudaError_t launch_quadrature_f64(int n, int npoint, const double *phi, long ld,
