@@ -241,8 +241,9 @@ int AuxiliaryBasis_get_nao(void *a);
 /* Device pointers of a grid's mirror: points (SoA), weights, Becke weights. */
 /* Moves the grid's centres (origin [ncenter][3], bohr): points rebuilt as at
  * construction (atomic_grid.cpp:12-51), device mirror rewritten in place,
- * Becke weights recomputed, Poisson tables dropped.  No counterpart in nAPMO
- * (it builds a new grid per geometry). */
+ * Becke weights recomputed, the Poisson plan's centres and pair lists rebuilt
+ * on its next use.  Synchronises the device.  No counterpart in nAPMO (it
+ * builds a new grid per geometry). */
 int napmo_grid_set_centers(void *grid, const double *origin);
 int napmo_grid_device_arrays(void *grid, double **x, double **y, double **z, double **w,
                              double **wb);
@@ -255,8 +256,10 @@ int napmo_gpu_becke_weights(int npoint, int ncenter, const double *x, const doub
  * points; replaces BasisSet_compute / BasisSet_deriv (basis_set.cpp:69-99). */
 int napmo_gpu_basis_values(void *basis, int npoint, const double *x, const double *y,
                            const double *z, double *phi, long ld, double *grad, void *stream);
-/* rho[p] = sum D[mu][nu] phi[mu][p] phi[nu][p]; phi [n][ld], ld >= npoint
- * rounded up to 128, zero padded; replaces the density of psi_hybrid.py:144-150. */
+/* rho[p] = sum D[mu][nu] phi[mu][p] phi[nu][p], D symmetric or not; phi [n][ld],
+ * ld >= npoint rounded up to 128, zero padded; replaces the density of
+ * psi_hybrid.py:144-150.  Above 64 functions it takes 8 n^2 bytes of
+ * stream-ordered scratch. */
 int napmo_gpu_density(int n, int npoint, const double *phi, long ld, const double *D,
                       double *rho, void *stream);
 /* F = phi diag(wv) psi^T (psi = phi if null), upper triangle mirrored;

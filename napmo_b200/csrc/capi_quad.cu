@@ -195,7 +195,8 @@ static int build_fp64_screening(FockPlan *p, double tol, cudaStream_t s) {
 }
 
 // The build chain of napmo_fock_plan_build (stream-ordered, no host
-// synchronisation, no allocation once the grid's Poisson plan exists).
+// synchronisation; once the grid's Poisson plan exists the only memory it takes
+// is the FP64 density's stream-ordered scratch).
 int fock_build(FockPlan *p, const double *D_dev, double q, const double *vext_dev, double *F_dev,
                double *rho_out, double *v_out, cudaStream_t s) {
   BeckeGrid *g = p->grid;

@@ -807,8 +807,9 @@ __global__ void identity_kernel(double *a, int ld) {
 // independent.  B200, substitution -> product: H2O 50 x 110 52 -> 13 us, C5H12
 // 75 x 194 81 -> 24, C12H26 100 x 302 111 -> 36, C20H42 215 -> 62, HCN 100 x 302
 // x 35 solves 151 -> 75.  It wins over the whole range it can take (H2O 10 x 50
-// 17 -> 5 us, 256 x 50 236 -> 60; C12H26 256 x 194 511 -> 143): kRadialOpMax is
-// where F and X come to fill the shared memory.
+// 17 -> 5 us, 256 x 50 236 -> 60; C12H26 256 x 194 511 -> 143; a batch of 64
+// uneven molecules, where hardly two atoms share an operator, 1873 -> 832):
+// kRadialOpMax is where F and X come to fill the shared memory.
 constexpr int kApplyCols = 32, kApplyThreads = 256;
 constexpr int kApplyLdf = kApplyCols + 4, kApplyLdx = kApplyCols + 1;
 

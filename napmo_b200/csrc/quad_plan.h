@@ -15,7 +15,11 @@ namespace napmo {
 
 constexpr int kQuadTile = 128;  // functions of a tile
 constexpr int kQuadStage = 16;  // points per stage
-constexpr int kSmallN = 64;     // whole triangle of fragments per warp up to this n
+// Whole triangle of fragments per warp up to this n.  B200, 66,000 points,
+// quadrature / density, us, against the tiled kernels: 40 functions 27 / 17 (35 /
+// 27), 48 27 / 17 (43 / 27), 49 to 64 31 / 25 (45 / 33), the last with 255
+// registers and 32 bytes spilled in the density; more functions do not fit.
+constexpr int kSmallN = 64;
 // row tiles of 16 that cover n <= kSmallN, and their upper-triangle fragments
 NAPMO_QUAD_FN constexpr int small_tiles(int n) { return (n + 15) / 16; }
 NAPMO_QUAD_FN constexpr int small_frags(int rt) { return rt * (rt + 1); }
@@ -46,7 +50,8 @@ NAPMO_QUAD_FN void quad_tile(int c, int t, int nblk, int &mb, int &nb) {
 
 // Cost of a stage of one tile: DMMA instructions per k8 step of the busiest
 // sub-partition (warps w and w + 4), plus the stage's fixed part (barrier and
-// copies, about 4 of them).
+// copies, about 4 of them; without it 310 functions x 1,147,600 points take 5.82
+// instead of 5.31 ms).
 inline int quad_tile_cost(int n, int nblk, int cls) {
   const bool ragged = cls == 1 || cls == 3;
   const int cols = ragged ? n - (nblk - 1) * kQuadTile : kQuadTile;
@@ -107,7 +112,8 @@ inline QuadPlan quad_plan_slots(int n, int npad, int slots, long *bound = nullpt
 
 // Slots: n <= 64 (a warp per chunk) four warps per SM; n > 64 (a CTA per slot,
 // one CTA per SM at these register counts) two full waves over the 148 SMs for
-// a single tile, four otherwise.
+// a single tile (110 functions x 200,000 points 171 us, 185 with four), four
+// otherwise (310 functions x 1,147,600 points 5.31 ms, 5.72 with two).
 inline int quad_default_slots(int n) { return n > kSmallN && n <= kQuadTile ? 2 * 148 : 4 * 148; }
 
 // Doubles of workspace for every range of at most npad points.

@@ -109,3 +109,22 @@ def test_captured_density_follows_its_input():
         graph.replay()
         ref, tol = _reference(D, phi[:, :npoint])
         assert bool(((rho - ref).abs() <= tol).all())
+
+
+def test_calls_on_two_streams_keep_their_own_folded_matrix():
+    import torch
+    from napmo_b200 import cext
+    n, npoint, ld = 145, 40000, 40064
+    phi = torch.zeros(n, ld, dtype=torch.float64, device='cuda')
+    phi[:, :npoint] = torch.randn(n, npoint, dtype=torch.float64, device='cuda')
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    Ds = [_matrix(n, 20 + k) for k in range(16)]
+    rhos = [torch.empty(npoint, dtype=torch.float64, device='cuda') for _ in Ds]
+    torch.cuda.synchronize()
+    for k, (D, rho) in enumerate(zip(Ds, rhos)):
+        cext.checked(cext.lib.napmo_gpu_density(n, npoint, phi.data_ptr(), ld, D.data_ptr(),
+                                                rho.data_ptr(), streams[k % 2].cuda_stream))
+    torch.cuda.synchronize()
+    for D, rho in zip(Ds, rhos):
+        ref, tol = _reference(D, phi[:, :npoint])
+        assert bool(((rho - ref).abs() <= tol).all())
