@@ -102,10 +102,14 @@ struct FockPlan {
   DevBuf<int> keep64, blocks64, groups64;
   int nblocks64 = 0, ngroups64 = 0;
   unsigned long long keep64_key = 0;
+  static std::atomic<int> live;  // Fock plans that exist
+  FockPlan() { ++live; }
   ~FockPlan() {
     if (i8) int8_plan_destroy(i8);
+    if (--live == 0) trim_call_scratch();
   }
 };
+std::atomic<int> FockPlan::live{0};
 
 // phi of the plan's basis on its grid, evaluated again when it was released
 // (napmo_fock_plan_release_phi); allocates, so it runs outside captures (the

@@ -53,6 +53,8 @@ struct DensBatchArg {      // density of one molecule
   int n, npoint;
 };
 size_t density_fold_doubles(int n);  // 0 where the kernel folds D itself
+// Returns what the density's scratch pools keep between calls to the driver.
+void trim_call_scratch();
 struct QuadBatchArg {      // quadrature of one molecule
   const double *phi;       // [n][ld]
   long ld;

@@ -783,16 +783,26 @@ __global__ void combine_weights_kernel(int npoint, const double *__restrict__ wb
 
 // Scratch of one call: stream-ordered, so safe with any streams and threads, and
 // a part of the graph when the stream is capturing.  From a pool of the
-// library's own per device, which keeps up to 64 MB between calls (the default
-// pool returns everything to the driver at each synchronisation).
+// library's own per device, which keeps up to 64 MB between calls until the last
+// Fock plan goes (trim_call_scratch).  The default pool returns everything to the
+// driver at each synchronisation, and so does one that keeps less than the blocks
+// it grows by (with 16 MB the C12H26 build took 14.6 ms instead of 13.5).
+struct ScratchPools {
+  std::mutex lock;
+  std::map<int, cudaMemPool_t> of;  // device -> pool
+};
+ScratchPools &scratch_pools() {
+  static ScratchPools *p = new ScratchPools;  // outlives every static plan
+  return *p;
+}
+
 cudaError_t call_scratch(void **p, size_t bytes, cudaStream_t s) {
-  static std::mutex lock;
-  static std::map<int, cudaMemPool_t> pools;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> hold(lock);
-  cudaMemPool_t &pool = pools[dev];
+  ScratchPools &pools = scratch_pools();
+  std::lock_guard<std::mutex> hold(pools.lock);
+  cudaMemPool_t &pool = pools.of[dev];
   if (!pool) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
@@ -854,6 +864,13 @@ cudaError_t launch_density_f64(int n, int npoint, const double *phi, long ld,
   e = cudaGetLastError();
   const cudaError_t ef = cudaFreeAsync(fold, s);
   return e != cudaSuccess ? e : ef;
+}
+
+void trim_call_scratch() {
+  ScratchPools &pools = scratch_pools();
+  std::lock_guard<std::mutex> hold(pools.lock);
+  for (auto &p : pools.of)
+    if (p.second) cudaMemPoolTrimTo(p.second, 0);
 }
 
 size_t density_fold_doubles(int n) { return n > kSmallN ? (size_t)n * fold_ld(n) : 0; }

@@ -128,3 +128,19 @@ def test_calls_on_two_streams_keep_their_own_folded_matrix():
     for D, rho in zip(Ds, rhos):
         ref, tol = _reference(D, phi[:, :npoint])
         assert bool(((rho - ref).abs() <= tol).all())
+
+
+def test_scratch_is_given_back_with_the_last_plan():
+    import gc
+    import torch
+    import napmo_b200 as nb
+    ms, grid = _systems()[2]
+    fb = nb.FockBuilder(grid, ms['e-']['basis'], 5)
+    for _ in range(3):  # each synchronisation may return memory; the results stay right
+        D = _matrix(fb.n, 7)
+        ref, tol = _reference(D, fb.phi()[:, :fb.npoint])
+        assert bool(((fb.density(D) - ref).abs() <= tol).all())
+    del fb
+    gc.collect()
+    again = nb.FockBuilder(grid, ms['e-']['basis'], 5)
+    assert bool(((again.density(D) - ref).abs() <= tol).all())
